@@ -144,8 +144,12 @@ private:
 constexpr int PERSIST_OK = 0, PERSIST_HALT = 1, PERSIST_TIMEOUT = 2;
 
 // The repair of one force evaluation (launch_repair's kernels), after the barrier that ends the force
-// pass: every thread of the grid takes the same decisions, from words that no block changes between
-// two barriers. On PERSIST_OK the rows, forces and counters are those of the repaired triangulation.
+// pass. Every thread of the grid takes the same decisions, each from words that are constant in the phase
+// that reads them: a block that read a word late and left alone would leave the others waiting. A star
+// that fails is recorded in `fail`, which the star phases write and the phases after them read; `halt`
+// is left to persist_end (the force pass sets it only for rows longer than its slots, which systems of
+// 16-slot rows do not have). On PERSIST_OK the rows, forces and counters are those of the repaired
+// triangulation.
 template <typename R, bool FORCES>
 CG_D int persist_repair(const VoroArgs &a, GridBarrier &gb, PersistWarp *wsm, Ctl *sum)
 {
@@ -168,9 +172,12 @@ CG_D int persist_repair(const VoroArgs &a, GridBarrier &gb, PersistWarp *wsm, Ct
     int r = 0;
     for (; r < R_MAX && nq > 0; ++r) {
         const int *queue = a.queue + (size_t)r * a.N;
-        for (int q = gw; q < nq; q += nw) star_one(a, ctl, r, queue, q, wsm[w].star, lane);
+        for (int q = gw; q < nq; q += nw) {
+            const int code = star_one(a, r, queue, q, wsm[w].star, lane);
+            if (code && lane == 0) atomicExch(&ctl->fail, code);
+        }
         if (!gb.wait()) return PERSIST_TIMEOUT;
-        if (vc->halt) return PERSIST_HALT;
+        if (vc->fail) return PERSIST_HALT;
         if (nq <= a.old_cap) {  // an even warp commits, the next one checks the same two slots
             for (int base = (gw >> 1) * (GPW / 2); base < nq; base += (nw >> 1) * (GPW / 2)) {
                 if ((w & 1) == 0)
@@ -190,11 +197,7 @@ CG_D int persist_repair(const VoroArgs &a, GridBarrier &gb, PersistWarp *wsm, Ct
         nq = vc->q_count[r + 1];
     }
     if (nq > 0) {  // the local repair did not converge: global rebuild
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            vc->need_global = 1;
-            vc->status = CG_ERR_TOPOLOGY;
-            vc->halt = 1;
-        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) vc->fail = CG_ERR_TOPOLOGY;
         return PERSIST_HALT;
     }
     return PERSIST_OK;
@@ -207,6 +210,7 @@ CG_D void ctl_reset(Ctl *c, int epoch)
     c->halt = 0;
     c->need_global = 0;
     c->status = 0;
+    c->fail = 0;
     c->n_flagged = 0;
     c->n_undec = 0;
     for (int r = 0; r <= R_MAX; ++r) c->q_count[r] = 0;
@@ -237,12 +241,15 @@ CG_D void persist_end(Ctl *c0, Ctl *cur, int st, int step)
     c0->step = step;
     if (st == PERSIST_OK) {
         ctl_reset(c0, c0->epoch > c1->epoch ? c0->epoch : c1->epoch);
-    } else if (cur == c1) {
-        c0->epoch = c1->epoch;
-        c0->need_global = c1->need_global;
-        c0->status = c1->status;
-        c0->halt = 1;
+        return;
     }
+    volatile Ctl *vc = cur;  // (other blocks wrote it)
+    const int fail = vc->fail;
+    c0->epoch = vc->epoch;
+    c0->need_global = fail ? 1 : vc->need_global;
+    c0->status = fail ? fail : vc->status;
+    __threadfence();
+    c0->halt = 1;
 }
 
 // The forces of the step are complete: F of cell c (from its fixed-point sums in the deterministic
@@ -412,7 +419,7 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_tail(PersistArgs p
     PersistWarp *wsm = reinterpret_cast<PersistWarp *>(persist_smem);
     VoroArgs a = p.a;
     Ctl *const c0 = p.a.ctl, *const c1 = c0 + 1;
-    if (c0->halt) return;  // uniform across the grid until this launch's first barrier or halt
+    if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
     a.ctl = c0 + (t & 1);
     GridBarrier gb = {p.bar + (t & 1), 0u, &s_ok, false};
     const int step = c0->step + t;  // (counted at the end of the call)

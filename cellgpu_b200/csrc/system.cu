@@ -1008,6 +1008,7 @@ static int reset_ctl_after_halt(cg_system *s)
     c.halt = 0;
     c.need_global = 0;
     c.status = 0;
+    c.fail = 0;
     c.n_flagged = 0;
     c.n_undec = 0;
     for (int r = 0; r <= R_MAX; ++r) c.q_count[r] = 0;

@@ -1340,8 +1340,9 @@ CG_D int flip_edit(const int *row, int z, int K, int4 h, int *out, int lane)
 }
 
 // exact star of the cell in queue slot q of `round` (whole warp); the result goes to the slot's
-// staging row, a failure halts the step
-CG_D void star_one(const VoroArgs &a, Ctl *ctl, int round, const int *queue, int q, StarSmem &S, int lane)
+// staging row. Returns 0, or the CG_* code of a star that needs a global rebuild (the step cannot
+// go on; the caller records it).
+CG_D int star_one(const VoroArgs &a, int round, const int *queue, int q, StarSmem &S, int lane)
 {
     volatile int *vm = &S.m;
     int c = queue[q];
@@ -1362,7 +1363,7 @@ CG_D void star_one(const VoroArgs &a, Ctl *ctl, int round, const int *queue, int
             if (lane < nz) a.stage_nbr[(size_t)q * a.K + lane] = S.out[lane];
             if (lane == 0) a.stage_nn[q] = nz;
             __syncwarp();
-            return;
+            return 0;
         }
         if (lane == 0 && h.x != 0) a.qhint[q].x = 0;  // the check then knows the row is a star
     }
@@ -1409,17 +1410,13 @@ CG_D void star_one(const VoroArgs &a, Ctl *ctl, int round, const int *queue, int
     StarFrame fr = {c, a.pos, in.Lx, in.Ly};
     int zs = warp_star(S.rel, S.cand, m, a.K, S.out, lane, fr);
     if (zs < 0) {
-        if (lane == 0) {
-            atomicExch(&ctl->need_global, 1);
-            atomicExch(&ctl->status, zs == -2 ? CG_ERR_CAPACITY : CG_ERR_TOPOLOGY);
-            atomicExch(&ctl->halt, 1);
-        }
         __syncwarp();
-        return;
+        return zs == -2 ? CG_ERR_CAPACITY : CG_ERR_TOPOLOGY;
     }
     if (lane < zs) a.stage_nbr[(size_t)q * a.K + lane] = S.out[lane];
     if (lane == 0) a.stage_nn[q] = zs;
     __syncwarp();
+    return 0;
 }
 
 template <int WPB>
@@ -1434,7 +1431,14 @@ __global__ void __launch_bounds__(WPB * 32, STAR_MINB) k_star_local(VoroArgs a)
     int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int gw = blockIdx.x * WPB + w, nw = gridDim.x * WPB;
     const int *queue = a.queue + (size_t)round * a.N;
-    for (int q = gw; q < nq; q += nw) star_one(a, ctl, round, queue, q, s_star[w], lane);
+    for (int q = gw; q < nq; q += nw) {
+        const int code = star_one(a, round, queue, q, s_star[w], lane);
+        if (code && lane == 0) {
+            atomicExch(&ctl->need_global, 1);
+            atomicExch(&ctl->status, code);
+            atomicExch(&ctl->halt, 1);
+        }
+    }
 }
 
 CG_D int row_find(const int *row, int z, int v)

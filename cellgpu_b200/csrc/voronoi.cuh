@@ -41,6 +41,7 @@ struct Ctl {
     int halt;                // sticky: a step could not complete on the device
     int need_global;         // a global retriangulation is required
     int status;              // CG_* code explaining halt
+    int fail;                // CG_* code of a cooperative launch's step that needs a global rebuild
     int n_flagged;           // cells flagged by the test of this step
     int n_undec;             // entries of VoroArgs::undec written by the test of this step
     int q_count[R_MAX + 1];  // per-round queue lengths
