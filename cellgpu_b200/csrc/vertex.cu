@@ -1476,11 +1476,12 @@ CG_D void vm_step_done(Ctl *ctl)
     if (!vc->halt) vc->step = vc->step + 1;
 }
 
-// The sweeps, a block per instance; with step, the last block to finish ends the step.
+// The sweeps, a block per instance; with step, the last block to finish ends the step. `halt` is not
+// asked for here: another block may set it meanwhile (a full cell row), and every instance still sweeps.
+// After a halt of an earlier launch the detection queued nothing, so the blocks find no candidates.
 __global__ void __launch_bounds__(256) k_vm_t1_replay(VertArgs a, int step)
 {
     extern __shared__ __align__(16) unsigned char t1_smem[];
-    if (a.ctl && a.ctl->halt) return;  // uniform
     t1_replay(a, a.ctl, blockIdx.x, t1_smem);
     if (!step) return;
     __syncthreads();
@@ -1502,7 +1503,7 @@ __global__ void __launch_bounds__(256) k_vm_t1(VertArgs a, int step)
     extern __shared__ __align__(16) unsigned char t1_smem[];
     __shared__ int s_last;
     Ctl *ctl = a.ctl;
-    if (ctl->halt) return;  // uniform
+    if (ctl->halt) return;  // uniform: set by an earlier launch, or by the last block after all have counted
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < a.Nv; v += gridDim.x * blockDim.x) vm_detect(a, v, nullptr);
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -329,7 +329,6 @@ static int vm_recover(cg_system *s, bool *recovered)
         CG_TRY(vm_grow_rows(s, s->vmax + 4));
         c.halt = 0;
         c.status = 0;
-        c.blocks_done = 0;  // (of a launch whose later blocks found the halt)
         CG_TRY(h2d(s, s->ctl, &c, sizeof(Ctl)));
         k_vm_t1_resume<<<s->n_inst, 32, T1_SMEM, s->stream>>>(vm_args(s));
         s->kernels_enqueued += 1;
