@@ -13,8 +13,8 @@
 // barriers; a repair round adds about 9 (star 1.3, commit and check 5, two barriers).
 //
 // The barrier is a counter in global memory that every block's first thread adds to and polls. All
-// blocks are resident (cooperative launch), and a wait gives up after PERSIST_WAIT_NS: the launch then
-// ends with CG_ERR_TIMEOUT in the control block.
+// blocks are resident (cooperative launch), and a wait gives up after wait_ns (PERSIST_WAIT_NS): the launch
+// then ends with CG_ERR_TIMEOUT in the control block, and the system is refused from then on.
 
 namespace cg {
 
@@ -37,6 +37,8 @@ struct PersistArgs {
     VoroArgs a;        // a.ctl: the control block; a.ctl[1]: the one of odd steps
     unsigned *bar;     // barrier arrivals, zero at launch
     int cluster;       // the grid is one thread-block cluster: its hardware barrier instead
+    int absent;        // arrivals that a barrier waits for and nothing makes (cg_inject_stall), else 0
+    unsigned long long wait_ns;  // after which a wait gives up
     int thread_form;   // the force pass in its thread-per-cell form
     const double *noise;  // steps x N normals, or null: drawn
     int steps;
@@ -62,13 +64,15 @@ struct GridBarrier {
     unsigned target;
     int *s_ok;
     bool cluster;
+    unsigned blocks;  // arrivals per barrier
+    unsigned long long wait_ns;
     CG_D void arrive()
     {
         if (cluster) {
             asm volatile("barrier.cluster.arrive.release;" ::: "memory");
             return;
         }
-        target += gridDim.x;
+        target += blocks;
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
@@ -100,7 +104,7 @@ struct GridBarrier {
             if (blockIdx.x == 0) last();
             return wait();
         }
-        target += gridDim.x + 1;  // one arrival more, when the last block is done
+        target += blocks + 1;  // one arrival more, when the last block is done
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
@@ -130,7 +134,7 @@ private:
             if ((i & 4095u) == 0) {
                 const unsigned long long t = now_ns();
                 if (t0 == 0) t0 = t;
-                else if (t - t0 > PERSIST_WAIT_NS) {
+                else if (t - t0 > wait_ns) {
                     ok = 0;
                     break;
                 }
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_steps(PersistArgs 
     VoroArgs a = p.a;
     Ctl *const c0 = p.a.ctl;
     if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
-    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0};
+    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0, gridDim.x + p.absent, p.wait_ns};
     const int step0 = c0->step;
     // a block's cells are contiguous, in whole warps' groups
     const int cpb = (a.N + gridDim.x * GPW - 1) / (gridDim.x * GPW) * GPW;
@@ -421,7 +425,7 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_tail(PersistArgs p
     Ctl *const c0 = p.a.ctl, *const c1 = c0 + 1;
     if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
     a.ctl = c0 + (t & 1);
-    GridBarrier gb = {p.bar + (t & 1), 0u, &s_ok, false};
+    GridBarrier gb = {p.bar + (t & 1), 0u, &s_ok, false, gridDim.x + p.absent, p.wait_ns};
     const int step = c0->step + t;  // (counted at the end of the call)
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     const bool lead = tid == 0;
@@ -544,7 +548,7 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_fire_voro(PersistArgs p
     VoroArgs a = p.a;
     Ctl *const c0 = p.a.ctl;
     if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
-    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0};
+    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0, gridDim.x + p.absent, p.wait_ns};
     const int step0 = c0->step;
     const int cpb = (a.N + gridDim.x * GPW - 1) / (gridDim.x * GPW) * GPW;
     const int lo = blockIdx.x * cpb, hi = min(a.N, lo + cpb);
@@ -670,7 +674,7 @@ static int persist_launch(cg_system *s, int *cluster, const void *kernel, void *
 {
     int grid = 0;
     CG_TRY(persist_grid(s, &grid));
-    *cluster = grid <= PERSIST_CLUSTER;
+    *cluster = grid <= PERSIST_CLUSTER && !s->stall_ns;  // (the hardware barrier has no limit to run out)
     CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -702,6 +706,8 @@ static int persist_args(cg_system *s, cg::PersistArgs &p)
     memset(&p, 0, sizeof(p));
     p.a = sys_args(s);
     p.bar = s->persist_bar;
+    p.absent = s->stall_ns ? 1 : 0;
+    p.wait_ns = s->stall_ns ? s->stall_ns : cg::PERSIST_WAIT_NS;
     p.excl = s->n_excl > 0 ? s->excl : nullptr;
     p.ext = s->ext_force;
     int grid = 0;

@@ -14,6 +14,8 @@ struct PersistVmArgs {
     VertArgs a;           // a.ctl: the control block; a.ctl[1]: the one of odd steps
     unsigned *bar;        // barrier arrivals, zero at launch
     int cluster;          // the grid is one thread-block cluster
+    int absent;           // as in PersistArgs
+    unsigned long long wait_ns;
     int kind;             // 0 Brownian, 1 self-propelled
     const double *noise;  // steps x (2 Nv or Nc) normals, or null: drawn
     int steps;
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_vm_steps(const __grid_c
     const VertArgs &a = p.a;
     Ctl *const c0 = p.a.ctl, *cur = c0;
     if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
-    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0};
+    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0, gridDim.x + p.absent, p.wait_ns};
     const int step0 = c0->step;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     const bool lead = tid == 0;
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_fire_vm(const __grid_co
     const VertArgs &a = p.a;
     Ctl *const c0 = p.a.ctl, *cur = c0;
     if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
-    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0};
+    GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0, gridDim.x + p.absent, p.wait_ns};
     const int step0 = c0->step;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     const bool lead = tid == 0;
@@ -214,6 +216,8 @@ static int persist_vm_args(cg_system *s, cg::PersistVmArgs &p)
     memset(&p, 0, sizeof(p));
     p.a = vm_args(s);
     p.bar = s->persist_bar;
+    p.absent = s->stall_ns ? 1 : 0;
+    p.wait_ns = s->stall_ns ? s->stall_ns : cg::PERSIST_WAIT_NS;
     return CG_OK;
 }
 

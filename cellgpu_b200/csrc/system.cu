@@ -315,6 +315,8 @@ struct cg_system {
     cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_consumed[2] = {nullptr, nullptr};
     int host_slot = 0;
     unsigned *persist_bar = nullptr;  // barrier counter of k_voro_steps
+    unsigned long long stall_ns = 0;  // cg_inject_stall
+    bool timed_out = false;           // a device wait gave up (refuse_timeout)
     // vertex model (model == CG_MODEL_VERTEX): pos/F are per vertex, AP/APpref/theta/motility per cell
     int Nv = 0, vmax = 0;
     int *vert_inst = nullptr, *vn = nullptr, *vcn = nullptr, *cvn = nullptr, *cv = nullptr;
@@ -1052,12 +1054,20 @@ static int grow_rows(cg_system *s)
     return cg_synchronize(s);
 }
 
+// A wait of a one-launch step gave up: some blocks had moved or cleared their cells and others had not,
+// so the system stays halted and its steps, minimisations and force evaluations are refused.
+static int refuse_timeout(cg_system *s)
+{
+    s->timed_out = true;
+    return set_err(CG_ERR_TIMEOUT, "a device wait gave up: the system's state is not usable any more");
+}
+
 static int recover(cg_system *s)
 {
     Ctl c;
     CG_TRY(read_ctl(s, c));
     if (!c.halt) return CG_OK;
-    if (c.status == CG_ERR_TIMEOUT) return set_err(CG_ERR_TIMEOUT, "a device wait gave up");
+    if (c.status == CG_ERR_TIMEOUT) return refuse_timeout(s);
     if (c.status == CG_ERR_CAPACITY) CG_TRY(grow_rows(s));
     CG_TRY(reset_ctl_after_halt(s));
     if (s->held) CG_CUDA(cudaMemsetAsync(s->held, 0, sizeof(int) * s->N, s->stream));
@@ -1080,6 +1090,7 @@ static int vm_enforce(cg_system *s);
 extern "C" int cg_compute_forces(cg_system *s)
 {
     if (!s) return set_err(CG_ERR_ARG, "null system");
+    if (s->timed_out) return refuse_timeout(s);
     if (s->model == CG_MODEL_VERTEX) return vm_compute_forces(s);
     if (!s->topology_valid) CG_TRY(triangulate_sys(s));
     int st = s->precision == CG_FP64 ? compute_forces_t<double>(s) : compute_forces_t<float>(s);
@@ -1489,6 +1500,15 @@ extern "C" int cg_poll(cg_system *s, int *steps_done, int *halted, int recover_i
     CG_TRY(read_status(s, steps_done, &h));
     if (halted) *halted = h;
     if (h && recover_if_halted) CG_TRY(recover(s));
+    return CG_OK;
+}
+
+// failure injection: the barriers of the system's cooperative launches wait for one block more than there
+// is, for at most `seconds` (0: as usual)
+extern "C" int cg_inject_stall(cg_system *s, double seconds)
+{
+    if (!s || !(seconds >= 0.0) || seconds > 10.0) return set_err(CG_ERR_ARG, "bad args");
+    s->stall_ns = (unsigned long long)(seconds * 1e9);
     return CG_OK;
 }
 

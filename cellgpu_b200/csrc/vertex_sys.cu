@@ -321,6 +321,7 @@ static int vm_recover(cg_system *s, bool *recovered)
         Ctl c;
         CG_TRY(read_ctl(s, c));
         if (!c.halt) return CG_OK;
+        if (c.status == CG_ERR_TIMEOUT) return refuse_timeout(s);
         std::vector<int> res(2 * (size_t)s->n_inst);
         CG_TRY(d2h(s, res.data(), s->t1_resume, sizeof(int) * res.size()));
         bool pending = false;

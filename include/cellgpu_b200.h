@@ -39,7 +39,7 @@ extern "C" {
 #define CG_ERR_ARG (-2)           /* invalid argument */
 #define CG_ERR_CAPACITY (-3)      /* a neighbour/vertex row exceeded its capacity; regrow needed */
 #define CG_ERR_TOPOLOGY (-4)      /* the triangulation could not be made consistent */
-#define CG_ERR_TIMEOUT (-5)       /* a bounded device wait gave up */
+#define CG_ERR_TIMEOUT (-5)       /* a bounded device wait gave up (the system is refused from then on) */
 #define CG_ERR_STATE (-6)         /* call not valid in the current state */
 
 /* precision modes */
@@ -217,6 +217,12 @@ int cg_spp_run(cg_system *sys, int n_steps, double dt, double mu, const double *
  * the remaining enqueued steps do nothing; cg_poll reports completed steps and recovers. */
 int cg_spp_enqueue(cg_system *sys, int n_steps, double dt, double mu);
 int cg_poll(cg_system *sys, int *steps_done, int *halted, int recover_if_halted);
+/* Failure injection, for tests of the error path: while seconds > 0, steps and FIRE iterations that run
+ * in cooperative launches wait at their barriers for a block that does not exist and give up after
+ * that long (at most 10 s; the default limit is 20 s and never met). The call that finds it returns
+ * CG_ERR_TIMEOUT; so do later steps, minimisations and force evaluations of the system, whose state is
+ * that of an unfinished step. Other systems and the CUDA context are not affected. */
+int cg_inject_stall(cg_system *sys, double seconds);
 /* One step through host buffers: host_noise (N normals) is copied in, the per-instance energies of
  * the step's force evaluation (the configuration at the start of the step) are copied out to
  * host_energy (may be NULL); returns when they are available. */
