@@ -190,14 +190,15 @@ extern "C" int cg_fire_advance(cg_system *s, const cg_fire_params *prm, int iter
         stopped = 0;
         for (auto &x : st) stopped += x.converged ? 1 : 0;
         if (stopped == s->n_inst || done >= iterations) break;
-        int todo = chunk;
         const bool vertex = persist_vm_ok(s, true);
-        if (vertex || persist_fire_ok(s)) {  // whole chunks of iterations in one launch
-            todo = std::min((iterations - done + chunk - 1) / chunk * chunk, PERSIST_FIRE_ITERS);
+        if (vertex || persist_fire_ok(s)) {
+            // the rest of the call's whole chunks in one launch, which ends early where it halts; every
+            // launch begins at least one iteration, so there are at most as many launches as iterations
+            const int left = (iterations - 1) / chunk * chunk + chunk - done;
+            int todo = std::min(left, PERSIST_FIRE_ITERS);
             CG_TRY(vertex ? enqueue_fire_vm(s, todo, f) : enqueue_fire_persistent(s, todo, f));
             CG_TRY(fire_after_launch(s, f, &todo));
             done += todo;
-            if (++rounds > prm->max_iterations / chunk + 64) return set_err(CG_ERR_STATE, "FIRE did not stop");
             continue;
         }
         // a graph of `chunk` iterations

@@ -85,3 +85,22 @@ def test_fire_iterations_rebuild(cglib, oracle, nx, ny):
     assert np.abs(d).max() < 1e-6 * np.abs(F).max()
     gnn, gnbr = b.topology()
     assert oracle.topology_mismatch(b.positions(), box, gnn, gnbr) == 0
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 32), (96, 100)])
+def test_fire_with_more_rebuilds_than_chunks(cglib, nx, ny):
+    """A time step so long that nearly every iteration needs a rebuild: 160 iterations, each of which may end
+    its launch, run through (10 chunks of 16; the oracle's run of the same parameters stays finite)."""
+    import cellgpu_b200 as cg
+
+    (pos,), (box,) = lattices([(nx, ny)])
+    n = len(pos)
+    b = cg.VoronoiBatch([n], [box])
+    b.set_positions(pos)
+    b.set_preferences(np.tile([1.0, 3.8], (n, 1)))
+    b.triangulate()
+    before = b.counters()["global_rebuilds"]
+    b.fire_minimize(cg.FireParams.defaults(dt=2.0, dt_max=2.0, dt_min=2.0, force_cutoff=1e-12, max_iterations=160))
+    assert b.counters()["global_rebuilds"] - before > 160 // 16 + 64
+    assert b.fire_state()[0][0] == 160
+    assert np.isfinite(b.positions()).all()
