@@ -314,6 +314,28 @@ CG_D void persist_energy(const VoroArgs &a, double *acc, int tid, int nt)
     }
 }
 
+// the sums to the host buffer, by one block; acc is left zeroed
+CG_D void energies_out(const VoroArgs &a, double *acc, double *host_out)
+{
+    for (int i = threadIdx.x; i < a.n_inst; i += blockDim.x)
+        host_out[i] =
+            __longlong_as_double((long long)atomicExch(reinterpret_cast<unsigned long long *>(acc + i), 0ull));
+    __threadfence_system();
+}
+
+// What a step that did not happen (it halted, or an earlier one had) leaves in the host buffer: the
+// energies of the stored areas and perimeters, as every other form does. The first block alone sums
+// them: no barrier is left to meet at, and halts are rare.
+template <typename R>
+CG_D void energies_of_halt(const VoroArgs &a, double *acc, double *host_out)
+{
+    if (blockIdx.x != 0) return;
+    persist_energy<R>(a, acc, threadIdx.x, blockDim.x);
+    __threadfence();
+    __syncthreads();
+    energies_out(a, acc, host_out);
+}
+
 // The fused force pass with the test over the block's cells [lo, hi): 8 lanes per cell, or a thread per
 // cell where a block has more cells than a few passes of its groups cover (FP64 with atomic sums).
 template <typename R, int FIX>
@@ -342,7 +364,10 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_steps(PersistArgs 
     PersistMove &mv = *reinterpret_cast<PersistMove *>(wsm + PERSIST_WPB);
     VoroArgs a = p.a;
     Ctl *const c0 = p.a.ctl;
-    if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
+    if (c0->halt) {  // uniform across the grid: set by an earlier launch only
+        if (p.acc) energies_of_halt<R>(a, p.acc, p.host_out);
+        return;
+    }
     GridBarrier gb = {p.bar, 0u, &s_ok, p.cluster != 0, gridDim.x + p.absent, p.wait_ns};
     const int step0 = c0->step;
     // a block's cells are contiguous, in whole warps' groups
@@ -401,12 +426,8 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_steps(PersistArgs 
         persist_timeout(c0, step0 + t);
         return;
     }
-    if (p.acc && st == PERSIST_OK && blockIdx.x == 0) {
-        for (int i = threadIdx.x; i < a.n_inst; i += blockDim.x)
-            p.host_out[i] = __longlong_as_double(
-                (long long)atomicExch(reinterpret_cast<unsigned long long *>(p.acc + i), 0ull));
-        __threadfence_system();
-    }
+    if (p.acc && st == PERSIST_OK && blockIdx.x == 0) energies_out(a, p.acc, p.host_out);
+    if (p.acc && st == PERSIST_HALT) energies_of_halt<R>(a, p.acc, p.host_out);
     if (lead) persist_end(c0, a.ctl, st, step0 + t);
 }
 
@@ -423,7 +444,10 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_tail(PersistArgs p
     PersistWarp *wsm = reinterpret_cast<PersistWarp *>(persist_smem);
     VoroArgs a = p.a;
     Ctl *const c0 = p.a.ctl, *const c1 = c0 + 1;
-    if (c0->halt) return;  // uniform across the grid: set by an earlier launch only
+    if (c0->halt) {  // uniform across the grid: set by an earlier launch only
+        if (p.acc && last) energies_of_halt<R>(a, p.acc, p.host_out);
+        return;
+    }
     a.ctl = c0 + (t & 1);
     GridBarrier gb = {p.bar + (t & 1), 0u, &s_ok, false, gridDim.x + p.absent, p.wait_ns};
     const int step = c0->step + t;  // (counted at the end of the call)
@@ -451,12 +475,8 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_voro_tail(PersistArgs p
         persist_timeout(c0, step);
         return;
     }
-    if (p.acc && st == PERSIST_OK && blockIdx.x == 0) {
-        for (int i = threadIdx.x; i < a.n_inst; i += blockDim.x)
-            p.host_out[i] = __longlong_as_double(
-                (long long)atomicExch(reinterpret_cast<unsigned long long *>(p.acc + i), 0ull));
-        __threadfence_system();
-    }
+    if (p.acc && st == PERSIST_OK && blockIdx.x == 0) energies_out(a, p.acc, p.host_out);
+    if (p.acc && last && st == PERSIST_HALT) energies_of_halt<R>(a, p.acc, p.host_out);
     if (lead) {
         persist_end(c0, a.ctl, st, st == PERSIST_OK ? step + 1 : step);
         if (st == PERSIST_HALT) c1->halt = 1;  // the force passes of the call's odd steps do nothing either
