@@ -223,6 +223,7 @@ extern "C" int cg_fire_advance(cg_system *s, const cg_fire_params *prm, int iter
             s->graphs.push_back(ge);
         }
         CG_CUDA(cudaGraphLaunch(exec, s->stream));
+        enqueued(s);
         s->kernels_enqueued += nk;
         CG_TRY(check_launch());
         CG_TRY(fire_after_launch(s, f, nullptr));

@@ -716,6 +716,7 @@ static int persist_launch(cg_system *s, int *cluster, const void *kernel, void *
         at.val.cooperative = 1;
     }
     CG_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+    enqueued(s);
     s->kernels_enqueued += 1;
     return CG_OK;
 }
@@ -773,6 +774,7 @@ static int split_steps(cg_system *s, cg::PersistArgs p)
             k_spp<R><<<nblk((s->N + 1) / 2, SPP_BLOCK), SPP_BLOCK, 0, s->stream>>>(
                 p.a, p.noise ? p.noise + (size_t)t * s->N : nullptr, p.dt, p.mu, last ? (uint32_t)-1 : (uint32_t)t, !last);
     }
+    enqueued(s);
     s->kernels_enqueued += (own_move ? 3 : 2) * (long long)p.steps;
     return check_launch();
 }

@@ -412,6 +412,7 @@ static int vm_run(cg_system *s, int kind, int n_steps, double dt, double mu, dou
                 s->graphs.push_back({gkind, todo, dt, mu, T, nullptr, exec, nk});
             }
             CG_CUDA(cudaGraphLaunch(exec, s->stream));
+            enqueued(s);
             s->kernels_enqueued += nk;
         }
         CG_TRY(check_launch());
