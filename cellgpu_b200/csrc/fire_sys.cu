@@ -181,6 +181,7 @@ extern "C" int cg_fire_advance(cg_system *s, const cg_fire_params *prm, int iter
 {
     if (!s || !prm || iterations < 0) return set_err(CG_ERR_ARG, "bad args");
     if (!s->fire_st) return set_err(CG_ERR_STATE, "cg_fire_begin first");
+    RunScope run(s);
     FireArgs f = fire_args(s, *prm);
     std::vector<FireInst> st(s->n_inst);
     const int chunk = 16;

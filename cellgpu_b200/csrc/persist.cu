@@ -656,14 +656,12 @@ constexpr int PERSIST_CLUSTER = 16;
 // groups and 29.1 with threads, 65536 43.9 and 35.7).
 constexpr int PERSIST_THREAD_CELLS = 192;
 
-// one block per SM at most, and no more blocks than the cells fill
-static int persist_grid(const cg_system *s, int *grid)
+// One block per SM at most, and no more blocks than the cells fill. Calls that run at the same time on
+// other systems take their share of the SMs: grids that fill the GPU would take turns.
+static int persist_grid(const cg_system *s)
 {
-    int dev = 0, sms = 0;
-    CG_CUDA(cudaGetDevice(&dev));
-    CG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    *grid = std::max(1, std::min(sms, nblk(s->N, cg::PERSIST_WPB * GPW)));
-    return CG_OK;
+    const int share = s->in_run ? std::max(1, s->sms / std::max(1, n_running[s->device & 63].load())) : s->sms;
+    return std::max(1, std::min(share, nblk(s->N, cg::PERSIST_WPB * GPW)));
 }
 
 // Cells above which k_spp integrates after the tail, at full occupancy (the tail has 16 warps per SM): a
@@ -678,22 +676,29 @@ static bool persist_any(const cg_system *s)
     return !(u && u[0] == '1') && s->K <= VG;
 }
 
-// Whether n steps of this system run as one cooperative launch.
-static bool persist_ok(const cg_system *s, int n)
+enum StepForm { STEP_GRAPH, STEP_ONE, STEP_TWO };  // the step graph, one launch, two launches per step
+
+// The form that n steps take. Single steps beside other systems' (host-driven ones on several streams) go
+// through the step graph, whose kernels overlap with theirs; two small systems also fit side by side.
+// us per round of single steps of M systems, one launch / graph:
+//   300 cells    M = 2  21 / 29    4  40 / 30    8   66 / 37
+//   4096 cells   M = 2  24 / 34    4  32 / 37    8   64 / 43
+//   16384 cells  M = 2  52 / 44    4 102 / 47    8  195 / 59
+static StepForm step_form(const cg_system *s, int n)
 {
-    if (!persist_any(s)) return false;
-    if (n == 1) return s->N <= (s->det ? PERSIST_MAX_SINGLE_FIX : PERSIST_MAX_SINGLE);
-    return s->N <= (persist_thread_ok(s) ? PERSIST_MAX_THREAD : PERSIST_MAX_CELLS);
+    if (!persist_any(s)) return STEP_GRAPH;
+    if (n == 1) {
+        const bool small = s->N <= (s->det ? PERSIST_MAX_SINGLE_FIX : PERSIST_MAX_SINGLE);
+        const int others = n_busy[s->device & 63].load() - (s->busy ? 1 : 0);
+        if (others > 0) return small && others == 1 && 2 * persist_grid(s) <= s->sms ? STEP_ONE : STEP_GRAPH;
+        return small ? STEP_ONE : STEP_TWO;
+    }
+    return s->N <= (persist_thread_ok(s) ? PERSIST_MAX_THREAD : PERSIST_MAX_CELLS) ? STEP_ONE : STEP_TWO;
 }
 
-// Whether they run as two launches per step.
-static bool split_ok(const cg_system *s, int n) { return persist_any(s) && !persist_ok(s, n); }
-
 // a cooperative launch, or one cluster (*cluster, an argument of the kernel, is set accordingly)
-static int persist_launch(cg_system *s, int *cluster, const void *kernel, void **args, size_t smem)
+static int persist_launch(cg_system *s, int grid, int *cluster, const void *kernel, void **args, size_t smem)
 {
-    int grid = 0;
-    CG_TRY(persist_grid(s, &grid));
     *cluster = grid <= PERSIST_CLUSTER && !s->stall_ns;  // (the hardware barrier has no limit to run out)
     CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg;
@@ -721,7 +726,7 @@ static int persist_launch(cg_system *s, int *cluster, const void *kernel, void *
     return CG_OK;
 }
 
-static int persist_args(cg_system *s, cg::PersistArgs &p)
+static int persist_args(cg_system *s, int grid, cg::PersistArgs &p)
 {
     if (!s->persist_bar) CG_TRY(dalloc(s, &s->persist_bar, 2));
     memset(&p, 0, sizeof(p));
@@ -731,8 +736,6 @@ static int persist_args(cg_system *s, cg::PersistArgs &p)
     p.wait_ns = s->stall_ns ? s->stall_ns : cg::PERSIST_WAIT_NS;
     p.excl = s->n_excl > 0 ? s->excl : nullptr;
     p.ext = s->ext_force;
-    int grid = 0;
-    CG_TRY(persist_grid(s, &grid));
     p.thread_form = persist_thread_ok(s) && s->N > PERSIST_THREAD_CELLS * grid;
     return CG_OK;
 }
@@ -746,19 +749,18 @@ static bool persist_fire_ok(const cg_system *s)
 static int enqueue_fire_persistent(cg_system *s, int n, cg::FireArgs f)
 {
     cg::PersistArgs p;
-    CG_TRY(persist_args(s, p));
+    const int grid = persist_grid(s);
+    CG_TRY(persist_args(s, grid, p));
     p.steps = n;
     void *args[] = {&p, &f};
-    return persist_launch(s, &p.cluster, (const void *)cg::k_fire_voro, args, cg::PERSIST_SMEM);
+    return persist_launch(s, grid, &p.cluster, (const void *)cg::k_fire_voro, args, cg::PERSIST_SMEM);
 }
 
 // the steps of p, each as its force pass and a cooperative launch for the rest (the sums are cleared)
 template <typename R>
-static int split_steps(cg_system *s, cg::PersistArgs p)
+static int split_steps(cg_system *s, int grid, cg::PersistArgs p)
 {
     const void *k = p.a.Ffix ? tail_kernel<R, 1>() : tail_kernel<R, 0>();
-    int grid = 0;
-    CG_TRY(persist_grid(s, &grid));
     CG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg::PERSIST_SMEM));
     CG_CUDA(cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), s->stream));
     const bool own_move = s->N > SPLIT_MOVE_CELLS && !p.a.Ffix && !p.excl;
@@ -782,11 +784,12 @@ static int split_steps(cg_system *s, cg::PersistArgs p)
 // n SPP steps, enqueued (noise: n x N normals on the device, or null; energy_dst: page-locked host
 // memory for the energies of the last step's force evaluation, e2e_acc allocated)
 template <typename R>
-static int enqueue_persistent(cg_system *s, int n, double dt, double mu, const double *noise,
+static int enqueue_persistent(cg_system *s, StepForm form, int n, double dt, double mu, const double *noise,
                               double *energy_dst = nullptr)
 {
     cg::PersistArgs p;
-    CG_TRY(persist_args(s, p));
+    const int grid = persist_grid(s);
+    CG_TRY(persist_args(s, grid, p));
     p.noise = noise;
     p.steps = n;
     p.dt = dt;
@@ -801,11 +804,11 @@ static int enqueue_persistent(cg_system *s, int n, double dt, double mu, const d
         CG_CUDA(cudaMemsetAsync(p.a.Ffix, 0, 2 * FIXF * sizeof(unsigned long long) * s->N, s->stream));
     else
         CG_CUDA(cudaMemsetAsync(s->F, 0, sizeof(double2) * s->N, s->stream));
-    if (persist_ok(s, n)) {
+    if (form == STEP_ONE) {
         void *args[] = {&p};
-        CG_TRY(persist_launch(s, &p.cluster, k, args, cg::PERSIST_SMEM));
+        CG_TRY(persist_launch(s, grid, &p.cluster, k, args, cg::PERSIST_SMEM));
     } else {
-        CG_TRY((split_steps<R>(s, p)));
+        CG_TRY((split_steps<R>(s, grid, p)));
     }
     if (fix_energy) {
         k_energy_to_host<R><<<nblk(s->N, 256), 256, 0, s->stream>>>(p.a, s->e2e_acc, s->e2e_done, energy_dst);

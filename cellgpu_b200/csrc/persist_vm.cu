@@ -237,7 +237,7 @@ static int enqueue_vm_persistent(cg_system *s, int kind, int n, double dt, doubl
     else
         CG_CUDA(cudaMemsetAsync(s->F, 0, sizeof(double2) * s->Nv, s->stream));
     void *args[] = {&p};
-    return persist_launch(s, &p.cluster, (const void *)cg::k_vm_steps, args, cg::PVM_SMEM);
+    return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_vm_steps, args, cg::PVM_SMEM);
 }
 
 // up to n FIRE iterations, enqueued (the FIRE state is set up and F holds the current forces)
@@ -247,5 +247,5 @@ static int enqueue_fire_vm(cg_system *s, int n, cg::FireArgs f)
     CG_TRY(persist_vm_args(s, p));
     p.steps = n;
     void *args[] = {&p, &f};
-    return persist_launch(s, &p.cluster, (const void *)cg::k_fire_vm, args, cg::PVM_SMEM);
+    return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_fire_vm, args, cg::PVM_SMEM);
 }

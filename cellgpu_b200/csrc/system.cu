@@ -1,6 +1,7 @@
 // cellgpu_b200 -- host side of the C ABI: kernel callers on caller memory, and the device-resident
 // batched system (cg_system). Built as one translation unit with the kernel files.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -258,6 +259,7 @@ struct cg_system {
     std::vector<Inst> h_inst;
     std::vector<int> h_cell_inst;
     cudaStream_t stream = 0;
+    int device = 0, sms = 0;
     uint64_t seed = 0x5eed;
     double KA = 1.0, KP = 1.0;
     size_t bytes = 0;
@@ -317,6 +319,7 @@ struct cg_system {
     unsigned *persist_bar = nullptr;  // barrier counter of k_voro_steps
     unsigned long long stall_ns = 0;  // cg_inject_stall
     bool busy = false;                // steps enqueued and not yet waited for
+    bool in_run = false;              // inside a call that runs steps or iterations and waits for them
     bool timed_out = false;           // a device wait gave up (refuse_timeout)
     // vertex model (model == CG_MODEL_VERTEX): pos/F are per vertex, AP/APpref/theta/motility per cell
     int Nv = 0, vmax = 0;
@@ -415,9 +418,29 @@ static int dalloc(cg_system *s, T **p, size_t count)
     return CG_OK;
 }
 
+// Per device, the systems with steps enqueued and not yet waited for, and those inside a call that runs
+// steps and waits for them. They share the GPU: the launch forms that hold whole SMs (persist.cu) look
+// at these counts, which change no result.
+static std::atomic<int> n_busy[64], n_running[64];
+
+static void mark(bool &flag, std::atomic<int> *count, const cg_system *s, bool on)
+{
+    if (flag == on) return;
+    flag = on;
+    count[s->device & 63] += on ? 1 : -1;
+}
+
+struct RunScope {
+    cg_system *s;
+    explicit RunScope(cg_system *sys) : s(sys) { mark(s->in_run, n_running, s, true); }
+    ~RunScope() { mark(s->in_run, n_running, s, false); }
+};
+
 // streams of a new system (before any allocation)
 static int sys_streams(cg_system *s)
 {
+    CG_CUDA(cudaGetDevice(&s->device));
+    CG_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device));
     CG_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking));
     CG_CUDA(cudaStreamCreateWithFlags(&s->body_stream, cudaStreamNonBlocking));
     s->stream = s->own_stream;
@@ -428,6 +451,7 @@ static int sys_streams(cg_system *s)
 static void sys_release(cg_system *s)
 {
     if (s->stream) cudaStreamSynchronize(s->stream);
+    mark(s->busy, n_busy, s, false);
     for (auto &g : s->graphs) release_graph(g);
     s->graphs.clear();
     cudaStream_t fs = s->own_stream;
@@ -657,7 +681,7 @@ extern "C" int cg_set_stream(cg_system *s, cudaStream_t stream)
 extern "C" cudaStream_t cg_get_stream(cg_system *s) { return s ? s->stream : nullptr; }
 
 // steps or iterations of the system are enqueued
-static void enqueued(cg_system *s) { s->busy = true; }
+static void enqueued(cg_system *s) { mark(s->busy, n_busy, s, true); }
 
 // Wait for them. A copy to or from pageable memory behind a launch of hundreds of steps would wait for
 // it inside the driver, with a lock that keeps every other thread from launching: four threads, each
@@ -667,7 +691,7 @@ static int settle(cg_system *s)
 {
     if (!s->busy) return CG_OK;
     CG_CUDA(cudaStreamSynchronize(s->stream));
-    s->busy = false;
+    mark(s->busy, n_busy, s, false);
     return CG_OK;
 }
 
@@ -675,7 +699,7 @@ extern "C" int cg_synchronize(cg_system *s)
 {
     if (!s) return set_err(CG_ERR_ARG, "null system");
     CG_CUDA(cudaStreamSynchronize(s->stream));
-    s->busy = false;
+    mark(s->busy, n_busy, s, false);
     return CG_OK;
 }
 
@@ -1335,8 +1359,9 @@ static int spp_run_t(cg_system *s, int n_steps, double dt, double mu, const doub
         int todo = chunk;
         while (todo > n_steps - done) todo >>= 1;
         const int left = n_steps - done;
-        if (!graph_only && (persist_ok(s, left) || split_ok(s, left)))
-            CG_TRY(enqueue_persistent<R>(s, std::min(left, persist_ok(s, left) ? 1024 : 128), dt, mu,
+        const StepForm form = graph_only ? STEP_GRAPH : step_form(s, left);
+        if (form != STEP_GRAPH)
+            CG_TRY(enqueue_persistent<R>(s, form, std::min(left, form == STEP_ONE ? 1024 : 128), dt, mu,
                                          noise ? noise + (size_t)done * s->N : nullptr));
         else if (noise)
             enqueue_spp_steps<R>(s, todo, dt, mu, noise + (size_t)done * s->N, true);
@@ -1357,8 +1382,10 @@ static int spp_run_t(cg_system *s, int n_steps, double dt, double mu, const doub
 static int enqueue_steps(cg_system *s, int n, double dt, double mu, const double *noise)
 {
     const bool fp64 = s->precision == CG_FP64;
-    if (persist_ok(s, n) || split_ok(s, n))
-        return fp64 ? enqueue_persistent<double>(s, n, dt, mu, noise) : enqueue_persistent<float>(s, n, dt, mu, noise);
+    const StepForm form = step_form(s, n);
+    if (form != STEP_GRAPH)
+        return fp64 ? enqueue_persistent<double>(s, form, n, dt, mu, noise)
+                    : enqueue_persistent<float>(s, form, n, dt, mu, noise);
     return fp64 ? enqueue_graph<double>(s, n, dt, mu, noise) : enqueue_graph<float>(s, n, dt, mu, noise);
 }
 
@@ -1421,7 +1448,8 @@ static int enqueue_energy_graph(cg_system *s, double dt, double mu, const double
         CG_TRY(dalloc(s, &s->e2e_acc, FIXW * (size_t)s->n_inst));  // zeroed; the kernel leaves it zeroed
         CG_TRY(dalloc(s, &s->e2e_done, 1));
     }
-    if (persist_ok(s, 1) || split_ok(s, 1)) return enqueue_persistent<R>(s, 1, dt, mu, noise, dst);
+    const StepForm form = step_form(s, 1);
+    if (form != STEP_GRAPH) return enqueue_persistent<R>(s, form, 1, dt, mu, noise, dst);
     for (auto &g : s->graphs)
         if (g.kind == 4 && g.dt == dt && g.mu == mu && g.noise == noise) {
             VoroArgs a = sys_args(s);
@@ -1565,6 +1593,7 @@ extern "C" int cg_spp_run(cg_system *s, int n_steps, double dt, double mu, const
 {
     if (!s || s->model != CG_MODEL_VORONOI || n_steps < 0) return set_err(CG_ERR_ARG, "bad args");
     if (!s->topology_valid) CG_TRY(triangulate_sys(s));
+    RunScope run(s);
     return s->precision == CG_FP64 ? spp_run_t<double>(s, n_steps, dt, mu, noise_dev)
                                    : spp_run_t<float>(s, n_steps, dt, mu, noise_dev);
 }

@@ -374,6 +374,7 @@ static void vm_enqueue_step(cg_system *s, int kind, int t, int n, double dt, dou
 static int vm_run(cg_system *s, int kind, int n_steps, double dt, double mu, double T, const double *noise)
 {
     if (!s->topology_valid) return set_err(CG_ERR_STATE, "vertex topology not set");
+    RunScope run(s);
     const int chunk = 32;  // graphs of 32, 16, ..., 1 steps: any n_steps reuses at most six graphs
     Ctl c0;
     CG_TRY(read_ctl(s, c0));
