@@ -627,10 +627,21 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_fire_voro(PersistArgs p
 //   N = 100000  49.2 / 45.6 / 58      63.5 / 53.6 / 64      57.1 / 47.5 / 58
 //   N = 262144  81.1 / 70.0 / 75.0      -  / 96.6 / 101       -  / 81.3 / 87.4
 // host steps: N = 300 19.7 / - / 29.4 and 24.3 / - / 27.7 (deterministic), 8192 31.7 / - / 38.4 and
-// 37.0 / - / 36.3, 65536 57.4 / 58.2 / 59.0, 131072 - / 72.2 / 76.0, 262144 - / 98.0 / 96.6; single
-// steps of 262144 cells with L2 flushed between them 92.7 against 95.6, host steps 93 against 101
+// 37.0 / - / 36.3, 65536 57.4 / 58.2 / 59.0
 constexpr int PERSIST_MAX_THREAD = 81920, PERSIST_MAX_CELLS = 30000;
 constexpr int PERSIST_MAX_SINGLE = 65536, PERSIST_MAX_SINGLE_FIX = 1024;
+// Single steps with fixed-point sums or in mixed precision above this many cells go through the step
+// graph: its integration runs beside the repair and at full occupancy, and these modes convert sums or
+// hold the force pass for longer. us per host step / single step / single step with L2 flushed, two
+// launches against the graph:
+//                deterministic                          mixed
+//   N =  66560    62 /  46 /  63    59 /  45 /  68       50 /  40 /  60    54 /  43 /  68
+//   N = 100000    77 /  58 /  76    71 /  59 /  82       65 /  51 /  70    62 /  50 /  72
+//   N = 180000   100 /  84 / 102    89 /  79 /  98       83 /  71 /  88    78 /  70 /  88
+//   N = 262144   125 / 107 / 125   110 / 101 / 121       96 /  87 / 106    95 /  86 / 102
+// FP64 with atomic sums: two launches at every size (100000 64 / 47 / 69 against 61 / 48 / 74, 262144 82 /
+// 68 / 86 against 82 / 70 / 90).
+constexpr int PERSIST_MAX_TWO_SINGLE = 90000;
 
 template <typename R, int FIX>
 static const void *persist_kernel() { return (const void *)cg::k_voro_steps<R, FIX>; }
@@ -666,7 +677,9 @@ static int persist_grid(const cg_system *s)
 
 // Cells above which k_spp integrates after the tail, at full occupancy (the tail has 16 warps per SM): a
 // 963507-cell ensemble 184 -> 167 us per step (the graph: 178), 400000 cells 92.4 -> 90.2, 262144 the same.
-constexpr int SPLIT_MOVE_CELLS = 300000;
+// Single steps from 200000: at 262144 cells with L2 flushed 86.0 -> 84.0 (warm 68.7 -> 70.0, host steps
+// 81.5 -> 81.1); at 180000 75.8 -> 73.8, 59.1 -> 60.4, 73.4 -> 73.5.
+constexpr int SPLIT_MOVE_CELLS = 300000, SPLIT_MOVE_SINGLE = 200000;
 
 // Whether steps can run without the step graph: 32-slot rows need the wide forms of the repair, and the
 // profiling form unrolls graphs.
@@ -691,7 +704,8 @@ static StepForm step_form(const cg_system *s, int n)
         const bool small = s->N <= (s->det ? PERSIST_MAX_SINGLE_FIX : PERSIST_MAX_SINGLE);
         const int others = n_busy[s->device & 63].load() - (s->busy ? 1 : 0);
         if (others > 0) return small && others == 1 && 2 * persist_grid(s) <= s->sms ? STEP_ONE : STEP_GRAPH;
-        return small ? STEP_ONE : STEP_TWO;
+        if (small) return STEP_ONE;
+        return s->N > PERSIST_MAX_TWO_SINGLE && (s->det || s->precision != CG_FP64) ? STEP_GRAPH : STEP_TWO;
     }
     return s->N <= (persist_thread_ok(s) ? PERSIST_MAX_THREAD : PERSIST_MAX_CELLS) ? STEP_ONE : STEP_TWO;
 }
@@ -763,7 +777,7 @@ static int split_steps(cg_system *s, int grid, cg::PersistArgs p)
     const void *k = p.a.Ffix ? tail_kernel<R, 1>() : tail_kernel<R, 0>();
     CG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg::PERSIST_SMEM));
     CG_CUDA(cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), s->stream));
-    const bool own_move = s->N > SPLIT_MOVE_CELLS && !p.a.Ffix && !p.excl;
+    const bool own_move = s->N > (p.steps == 1 ? SPLIT_MOVE_SINGLE : SPLIT_MOVE_CELLS) && !p.a.Ffix && !p.excl;
     for (int t = 0; t < p.steps; ++t) {
         VoroArgs a = p.a;
         a.ctl = p.a.ctl + (t & 1);
