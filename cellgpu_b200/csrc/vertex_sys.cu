@@ -270,10 +270,20 @@ static int vm_compute_forces(cg_system *s)
     return cg_synchronize(s);
 }
 
-// T1 detection and sweep; with step, the last kernel also ends the step
+// T1 detection and sweep; with step, the last kernel also ends the step. For a single instance both can be
+// one launch, which saves a kernel boundary but whose blocks each reserve the sweep's shared memory, so
+// the detection runs at a block per SM and other systems' kernels find no room beside it. us per step or
+// iteration, one launch / two, of one system and of eight in eight threads:
+//   Brownian steps     9000 cells 15.8 / 17.5 and  30 /  28    16384 18.5 / 20.4 and  49 /  41
+//                     45000       30.1 / 30.1 and 124 /  99    60000 36.0 / 35.9 and 166 / 136
+//   FIRE iterations    4096       18.0 / 18.2 and  24 /  23     9000 19.6 / 19.4 and  33 /  30
+//                     16384       19.5 / 19.0 and  53 /  41    60000 34.6 / 31.1 and 187 / 154
+// (a FIRE from a random dual, with flips in every sweep, 4096 cells: 32.5 / 33.9)
+constexpr int T1_ONE_STEP = 40000, T1_ONE_SWEEP = 8192;
+
 static void vm_launch_t1(cg_system *s, const VertArgs &a, int step = 0)
 {
-    if (s->n_inst == 1) {
+    if (s->n_inst == 1 && s->N <= (step ? T1_ONE_STEP : T1_ONE_SWEEP)) {
         k_vm_t1<<<std::min(nblk(s->Nv, 256), 148), 256, T1_SMEM, s->stream>>>(a, step);
         s->kernels_enqueued += 1;
         return;
