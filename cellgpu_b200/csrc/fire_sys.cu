@@ -197,7 +197,9 @@ extern "C" int cg_fire_advance(cg_system *s, const cg_fire_params *prm, int iter
             // launch begins at least one iteration, so there are at most as many launches as iterations
             const int left = (iterations - 1) / chunk * chunk + chunk - done;
             int todo = std::min(left, PERSIST_FIRE_ITERS);
-            CG_TRY(vertex ? enqueue_fire_vm(s, todo, f) : enqueue_fire_persistent(s, todo, f));
+            const int launched = vertex ? enqueue_fire_vm(s, todo, f) : enqueue_fire_persistent(s, todo, f);
+            if (launched == PERSIST_REFUSED) continue;  // (by graphs)
+            CG_TRY(launched);
             CG_TRY(fire_after_launch(s, f, &todo));
             done += todo;
             continue;

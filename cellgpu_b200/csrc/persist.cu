@@ -681,12 +681,12 @@ static int persist_grid(const cg_system *s)
 // 81.5 -> 81.1); at 180000 75.8 -> 73.8, 59.1 -> 60.4, 73.4 -> 73.5.
 constexpr int SPLIT_MOVE_CELLS = 300000, SPLIT_MOVE_SINGLE = 200000;
 
-// Whether steps can run without the step graph: 32-slot rows need the wide forms of the repair, and the
+// Whether steps can run without the step graph: the device takes the launches, 32-slot rows need the wide forms of the repair, and the
 // profiling form unrolls graphs.
 static bool persist_any(const cg_system *s)
 {
     const char *u = getenv("CG_GRAPH_UNROLLED");
-    return !(u && u[0] == '1') && s->K <= VG;
+    return !(u && u[0] == '1') && s->K <= VG && !s->coop_refused;
 }
 
 enum StepForm { STEP_GRAPH, STEP_ONE, STEP_TWO };  // the step graph, one launch, two launches per step
@@ -710,9 +710,28 @@ static StepForm step_form(const cg_system *s, int n)
     return s->N <= (persist_thread_ok(s) ? PERSIST_MAX_THREAD : PERSIST_MAX_CELLS) ? STEP_ONE : STEP_TWO;
 }
 
-// a cooperative launch, or one cluster (*cluster, an argument of the kernel, is set accordingly)
+// A launch that the device refuses (fewer SMs than the grid for this process, no room for a cluster in any
+// GPC): nothing of it ran, and the system's steps go by graphs from then on.
+constexpr int PERSIST_REFUSED = 1;
+
+static bool launch_refused(cudaError_t e)
+{
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources ||
+           e == cudaErrorInvalidConfiguration || e == cudaErrorInvalidClusterSize || e == cudaErrorNotSupported;
+}
+
+static int persist_refused(cg_system *s)
+{
+    cudaGetLastError();  // (not sticky)
+    s->coop_refused = true;
+    return PERSIST_REFUSED;
+}
+
+// A cooperative launch, or one cluster where the grid is small and a GPC has room for it (*cluster, an
+// argument of the kernel, is set accordingly).
 static int persist_launch(cg_system *s, int grid, int *cluster, const void *kernel, void **args, size_t smem)
 {
+    if (s->inject_refusal) grid = 4 * s->sms;  // (a block takes an SM)
     *cluster = grid <= PERSIST_CLUSTER && !s->stall_ns;  // (the hardware barrier has no limit to run out)
     CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg;
@@ -724,17 +743,26 @@ static int persist_launch(cg_system *s, int grid, int *cluster, const void *kern
     cudaLaunchAttribute at;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
+    cudaError_t e = cudaSuccess;
     if (*cluster) {
         CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = grid;
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    } else {
+        e = cudaLaunchKernelExC(&cfg, kernel, args);
+        if (launch_refused(e)) {
+            cudaGetLastError();
+            *cluster = 0;
+        }
+    }
+    if (!*cluster) {
         CG_CUDA(cudaMemsetAsync(s->persist_bar, 0, sizeof(unsigned), s->stream));
         at.id = cudaLaunchAttributeCooperative;
         at.val.cooperative = 1;
+        e = cudaLaunchKernelExC(&cfg, kernel, args);
+        if (launch_refused(e)) return persist_refused(s);
     }
-    CG_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+    CG_CUDA(e);
     enqueued(s);
     s->kernels_enqueued += 1;
     return CG_OK;
@@ -759,7 +787,7 @@ static bool persist_fire_ok(const cg_system *s)
     return s->model == CG_MODEL_VORONOI && !s->det && s->N <= PERSIST_MAX_FIRE && persist_any(s);
 }
 
-// up to n FIRE iterations, enqueued (the FIRE state is set up and F holds the current forces)
+// up to n FIRE iterations, enqueued, or PERSIST_REFUSED (the FIRE state is set up and F holds the current forces)
 static int enqueue_fire_persistent(cg_system *s, int n, cg::FireArgs f)
 {
     cg::PersistArgs p;
@@ -775,6 +803,7 @@ template <typename R>
 static int split_steps(cg_system *s, int grid, cg::PersistArgs p)
 {
     const void *k = p.a.Ffix ? tail_kernel<R, 1>() : tail_kernel<R, 0>();
+    if (s->inject_refusal) grid = 4 * s->sms;
     CG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg::PERSIST_SMEM));
     CG_CUDA(cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), s->stream));
     const bool own_move = s->N > (p.steps == 1 ? SPLIT_MOVE_SINGLE : SPLIT_MOVE_CELLS) && !p.a.Ffix && !p.excl;
@@ -784,8 +813,16 @@ static int split_steps(cg_system *s, int grid, cg::PersistArgs p)
         launch_groups<R, true, true>(a, s->N, s->stream, s->tune_force);
         int last = t + 1 == p.steps, move = !own_move;
         void *args[] = {&p, &t, &last, &move};
-        CG_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(cg::PERSIST_WPB * 32), args, cg::PERSIST_SMEM,
-                                            s->stream));
+        const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(cg::PERSIST_WPB * 32), args,
+                                                          cg::PERSIST_SMEM, s->stream);
+        if (t == 0 && launch_refused(e)) {  // the force pass has run: take its queues back
+            Ctl c;
+            persist_refused(s);
+            CG_TRY(read_ctl(s, c));
+            if (!c.halt) CG_TRY(clear_queues(s));  // (halted before: it did nothing)
+            return PERSIST_REFUSED;
+        }
+        CG_CUDA(e);
         if (own_move)  // (the step is counted at the end of the call, by its last tail)
             k_spp<R><<<nblk((s->N + 1) / 2, SPP_BLOCK), SPP_BLOCK, 0, s->stream>>>(
                 p.a, p.noise ? p.noise + (size_t)t * s->N : nullptr, p.dt, p.mu, last ? (uint32_t)-1 : (uint32_t)t, !last);
@@ -795,7 +832,7 @@ static int split_steps(cg_system *s, int grid, cg::PersistArgs p)
     return check_launch();
 }
 
-// n SPP steps, enqueued (noise: n x N normals on the device, or null; energy_dst: page-locked host
+// n SPP steps, enqueued, or PERSIST_REFUSED (noise: n x N normals on the device, or null; energy_dst: page-locked host
 // memory for the energies of the last step's force evaluation, e2e_acc allocated)
 template <typename R>
 static int enqueue_persistent(cg_system *s, StepForm form, int n, double dt, double mu, const double *noise,
@@ -820,9 +857,11 @@ static int enqueue_persistent(cg_system *s, StepForm form, int n, double dt, dou
         CG_CUDA(cudaMemsetAsync(s->F, 0, sizeof(double2) * s->N, s->stream));
     if (form == STEP_ONE) {
         void *args[] = {&p};
-        CG_TRY(persist_launch(s, grid, &p.cluster, k, args, cg::PERSIST_SMEM));
+        const int st = persist_launch(s, grid, &p.cluster, k, args, cg::PERSIST_SMEM);
+        if (st) return st;
     } else {
-        CG_TRY((split_steps<R>(s, grid, p)));
+        const int st = split_steps<R>(s, grid, p);
+        if (st) return st;
     }
     if (fix_energy) {
         k_energy_to_host<R><<<nblk(s->N, 256), 256, 0, s->stream>>>(p.a, s->e2e_acc, s->e2e_done, energy_dst);

@@ -207,7 +207,7 @@ constexpr int PERSIST_VM_MAX = 2048;
 
 static bool persist_vm_ok(const cg_system *s, bool fire)
 {
-    return s->model == CG_MODEL_VERTEX && s->vmax <= VM_ROW_G && s->N <= PERSIST_VM_MAX && !(fire && s->det);
+    return s->model == CG_MODEL_VERTEX && !s->coop_refused && s->vmax <= VM_ROW_G && s->N <= PERSIST_VM_MAX && !(fire && s->det);
 }
 
 static int persist_vm_args(cg_system *s, cg::PersistVmArgs &p)
@@ -221,7 +221,7 @@ static int persist_vm_args(cg_system *s, cg::PersistVmArgs &p)
     return CG_OK;
 }
 
-// n steps, enqueued (noise: n steps' normals on the device, or null)
+// n steps, enqueued, or PERSIST_REFUSED (noise: n steps' normals on the device, or null)
 static int enqueue_vm_persistent(cg_system *s, int kind, int n, double dt, double mu, double T, const double *noise)
 {
     cg::PersistVmArgs p;
@@ -240,7 +240,7 @@ static int enqueue_vm_persistent(cg_system *s, int kind, int n, double dt, doubl
     return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_vm_steps, args, cg::PVM_SMEM);
 }
 
-// up to n FIRE iterations, enqueued (the FIRE state is set up and F holds the current forces)
+// up to n FIRE iterations, enqueued, or PERSIST_REFUSED (the FIRE state is set up and F holds the current forces)
 static int enqueue_fire_vm(cg_system *s, int n, cg::FireArgs f)
 {
     cg::PersistVmArgs p;

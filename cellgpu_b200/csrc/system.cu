@@ -317,7 +317,9 @@ struct cg_system {
     cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_consumed[2] = {nullptr, nullptr};
     int host_slot = 0;
     unsigned *persist_bar = nullptr;  // barrier counter of k_voro_steps
+    bool coop_refused = false;        // the device refused a cooperative launch: graphs from then on
     unsigned long long stall_ns = 0;  // cg_inject_stall
+    bool inject_refusal = false;      // cg_inject_refusal
     bool busy = false;                // steps enqueued and not yet waited for
     bool in_run = false;              // inside a call that runs steps or iterations and waits for them
     bool timed_out = false;           // a device wait gave up (refuse_timeout)
@@ -1097,6 +1099,15 @@ static int grow_rows(cg_system *s)
     return cg_synchronize(s);
 }
 
+// forget the halt and what the step's force pass queued, claimed and held
+static int clear_queues(cg_system *s)
+{
+    CG_TRY(reset_ctl_after_halt(s));
+    if (s->held) CG_CUDA(cudaMemsetAsync(s->held, 0, sizeof(int) * s->N, s->stream));
+    if (s->nclaim) CG_CUDA(cudaMemsetAsync(s->nclaim, 0, sizeof(int) * s->N, s->stream));
+    return CG_OK;
+}
+
 // A wait of a one-launch step gave up: some blocks had moved or cleared their cells and others had not,
 // so the system stays halted and its steps, minimisations and force evaluations are refused.
 static int refuse_timeout(cg_system *s)
@@ -1112,9 +1123,7 @@ static int recover(cg_system *s)
     if (!c.halt) return CG_OK;
     if (c.status == CG_ERR_TIMEOUT) return refuse_timeout(s);
     if (c.status == CG_ERR_CAPACITY) CG_TRY(grow_rows(s));
-    CG_TRY(reset_ctl_after_halt(s));
-    if (s->held) CG_CUDA(cudaMemsetAsync(s->held, 0, sizeof(int) * s->N, s->stream));
-    if (s->nclaim) CG_CUDA(cudaMemsetAsync(s->nclaim, 0, sizeof(int) * s->N, s->stream));
+    CG_TRY(clear_queues(s));
     return triangulate_sys(s);
 }
 
@@ -1360,10 +1369,13 @@ static int spp_run_t(cg_system *s, int n_steps, double dt, double mu, const doub
         while (todo > n_steps - done) todo >>= 1;
         const int left = n_steps - done;
         const StepForm form = graph_only ? STEP_GRAPH : step_form(s, left);
+        int st = PERSIST_REFUSED;
         if (form != STEP_GRAPH)
-            CG_TRY(enqueue_persistent<R>(s, form, std::min(left, form == STEP_ONE ? 1024 : 128), dt, mu,
-                                         noise ? noise + (size_t)done * s->N : nullptr));
-        else if (noise)
+            st = enqueue_persistent<R>(s, form, std::min(left, form == STEP_ONE ? 1024 : 128), dt, mu,
+                                       noise ? noise + (size_t)done * s->N : nullptr);
+        if (st < 0) return st;
+        if (st != PERSIST_REFUSED) {
+        } else if (noise)
             enqueue_spp_steps<R>(s, todo, dt, mu, noise + (size_t)done * s->N, true);
         else
             CG_TRY(enqueue_graph<R>(s, todo, dt, mu, nullptr));
@@ -1383,9 +1395,11 @@ static int enqueue_steps(cg_system *s, int n, double dt, double mu, const double
 {
     const bool fp64 = s->precision == CG_FP64;
     const StepForm form = step_form(s, n);
-    if (form != STEP_GRAPH)
-        return fp64 ? enqueue_persistent<double>(s, form, n, dt, mu, noise)
-                    : enqueue_persistent<float>(s, form, n, dt, mu, noise);
+    if (form != STEP_GRAPH) {
+        const int st = fp64 ? enqueue_persistent<double>(s, form, n, dt, mu, noise)
+                            : enqueue_persistent<float>(s, form, n, dt, mu, noise);
+        if (st != PERSIST_REFUSED) return st;
+    }
     return fp64 ? enqueue_graph<double>(s, n, dt, mu, noise) : enqueue_graph<float>(s, n, dt, mu, noise);
 }
 
@@ -1449,7 +1463,10 @@ static int enqueue_energy_graph(cg_system *s, double dt, double mu, const double
         CG_TRY(dalloc(s, &s->e2e_done, 1));
     }
     const StepForm form = step_form(s, 1);
-    if (form != STEP_GRAPH) return enqueue_persistent<R>(s, form, 1, dt, mu, noise, dst);
+    if (form != STEP_GRAPH) {
+        const int st = enqueue_persistent<R>(s, form, 1, dt, mu, noise, dst);
+        if (st != PERSIST_REFUSED) return st;
+    }
     for (auto &g : s->graphs)
         if (g.kind == 4 && g.dt == dt && g.mu == mu && g.noise == noise) {
             VoroArgs a = sys_args(s);
@@ -1560,6 +1577,14 @@ extern "C" int cg_inject_stall(cg_system *s, double seconds)
 {
     if (!s || !(seconds >= 0.0) || seconds > 10.0) return set_err(CG_ERR_ARG, "bad args");
     s->stall_ns = (unsigned long long)(seconds * 1e9);
+    return CG_OK;
+}
+
+// failure injection: cooperative launches ask for more blocks than the GPU holds
+extern "C" int cg_inject_refusal(cg_system *s, int on)
+{
+    if (!s) return set_err(CG_ERR_ARG, "null system");
+    s->inject_refusal = on != 0;
     return CG_OK;
 }
 

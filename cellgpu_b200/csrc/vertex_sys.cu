@@ -394,8 +394,10 @@ static int vm_run(cg_system *s, int kind, int n_steps, double dt, double mu, dou
         while (todo > n_steps - done) todo >>= 1;
         if (persist_vm_ok(s, false)) {
             const size_t per_step = kind == 0 ? 2 * (size_t)s->Nv : (size_t)s->N;
-            CG_TRY(enqueue_vm_persistent(s, kind, std::min(n_steps - done, 1024), dt, mu, T,
-                                         noise ? noise + (size_t)done * per_step : nullptr));
+            const int st = enqueue_vm_persistent(s, kind, std::min(n_steps - done, 1024), dt, mu, T,
+                                                 noise ? noise + (size_t)done * per_step : nullptr);
+            if (st == PERSIST_REFUSED) continue;  // (by graphs)
+            CG_TRY(st);
         } else if (noise) {
             const size_t per_step = kind == 0 ? 2 * (size_t)s->Nv : (size_t)s->N;
             for (int t = 0; t < todo; ++t)

@@ -223,6 +223,10 @@ int cg_poll(cg_system *sys, int *steps_done, int *halted, int recover_if_halted)
  * CG_ERR_TIMEOUT; so do later steps, minimisations and force evaluations of the system, whose state is
  * that of an unfinished step. Other systems and the CUDA context are not affected. */
 int cg_inject_stall(cg_system *sys, double seconds);
+/* Failure injection: while on, the system's cooperative launches ask for more blocks than the GPU holds,
+ * so the driver refuses them as it does where a process has only some of the SMs. The system's steps
+ * and iterations then run by graphs. */
+int cg_inject_refusal(cg_system *sys, int on);
 /* One step through host buffers: host_noise (N normals) is copied in, the per-instance energies of
  * the step's force evaluation (the configuration at the start of the step) are copied out to
  * host_energy (may be NULL); returns when they are available. */
