@@ -304,7 +304,7 @@ struct cg_system {
     std::vector<GraphEntry> graphs;
     long long kernels_enqueued = 0;  // kernels of this library launched for this system
     double *noise_buf = nullptr;     // staging for host-supplied noise (one step)
-    double *draw_buf = nullptr;      // velocities and next directors of the step (k_spp_turn), 3 N
+    double *draw_buf = nullptr;      // next directors of the step (k_spp_turn)
     // deterministic force sums (cg_set_deterministic): fixed-point accumulator, 4 words per cell
     int det = 0;
     unsigned long long *Ffix = nullptr;
@@ -531,7 +531,7 @@ static size_t voronoi_bytes(int N, int K, int n_bins, int n_inst, int precision)
     size_t per_cell = 4 /*cell_inst*/ + 4 /*held*/ + 4 /*undec*/ + 16 * 3 /*pos, motility, APpref*/ + 8 /*theta*/ + real2 /*AP*/ + 16 /*F*/ +
                       4 + 4 * (size_t)K /*nn, nbr*/ + 4 /*mark*/ + 4 * (R_MAX + 1) /*queue*/ + 4 +
                       4 * (size_t)K /*stage*/ + 4 * 2 /*qslot*/ + 16 /*qhint*/ + 4 /*nclaim*/ + 4 * 3 + 16 /*cell list*/ +
-                      8 + 24 /*noise staging, staged integration*/;
+                      8 + 8 /*noise staging, staged integration*/;
     return per_cell * (size_t)N + (size_t)std::min(N, OLD_ROWS) * 4 * (K + 1) /*old rows*/ + (size_t)n_bins * 8 +
            (size_t)n_inst * (sizeof(Inst) + 16) + 4096;
 }
@@ -617,7 +617,7 @@ extern "C" int cg_voronoi_create(int n_inst, const int *N, const double *box, in
         s->d_zsum = reinterpret_cast<unsigned long long *>(s->d_status + 4);
         if ((st = dalloc(s, &s->d_energy, n_inst))) break;
         if ((st = dalloc(s, &s->noise_buf, Nt))) break;
-        if ((st = dalloc(s, &s->draw_buf, 3 * (size_t)Nt))) break;
+        if ((st = dalloc(s, &s->draw_buf, Nt))) break;
         size_t tmpb = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tmpb, s->bin_count, s->bin_start, s->n_bins + 1);
         s->scan_tmp_bytes = tmpb;

@@ -2249,24 +2249,23 @@ __global__ void k_fix_forces(VoroArgs a)
 }
 
 // What the step's integration can know before its forces: every cell's velocity and its director after
-// the step, into turn (N velocities, then N directors), from the given normals or the ones drawn for the
-// current step. The step graph runs this beside the repair rounds, which leave most of the GPU idle, so
-// that the kernel after them (k_spp_shift) only moves the cells: the integration took 9.3 us of a
-// 262144-cell step and 23 us of a 963507-cell one, most of it in sincos and atan2.
+// the step, from the given normals or the ones drawn for the current step. The velocities are kept in
+// bin_pos, which only the global triangulation uses (never between this kernel and the shift), the
+// directors in turn[N]. The step graph runs this beside the repair rounds, which leave most of the GPU
+// idle, so that the kernel after them (k_spp_shift) only moves the cells: the integration took 9.3 us of
+// a 262144-cell step and 23 us of a 963507-cell one, most of it in sincos and atan2.
 __global__ void k_spp_turn(VoroArgs a, const double *noise, double dt, double *turn)
 {
     const int c0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (c0 >= a.N) return;
     const bool two = c0 + 1 < a.N;
     const double2 xi = noise ? make_double2(noise[c0], two ? noise[c0 + 1] : 0.0) : pair_draw(a, c0, (uint32_t)a.ctl->step);
-    double2 *v = reinterpret_cast<double2 *>(turn);
-    double *th = turn + 2 * (size_t)a.N;
     double2 w;
-    th[c0] = spp_turn(a, c0, xi.x, dt, w.x, w.y);
-    v[c0] = w;
+    turn[c0] = spp_turn(a, c0, xi.x, dt, w.x, w.y);
+    a.bin_pos[c0] = w;
     if (two) {
-        th[c0 + 1] = spp_turn(a, c0 + 1, xi.y, dt, w.x, w.y);
-        v[c0 + 1] = w;
+        turn[c0 + 1] = spp_turn(a, c0 + 1, xi.y, dt, w.x, w.y);
+        a.bin_pos[c0 + 1] = w;
     }
 }
 
@@ -2274,8 +2273,8 @@ __global__ void k_spp_turn(VoroArgs a, const double *noise, double dt, double *t
 CG_D void spp_staged(const VoroArgs &a, int c, const double *turn, double dt, double mu, int clear)
 {
     double2 *F = reinterpret_cast<double2 *>(a.F);
-    const double2 f = F[c], v = reinterpret_cast<const double2 *>(turn)[c];
-    const double th = turn[2 * (size_t)a.N + c];
+    const double2 f = F[c], v = a.bin_pos[c];
+    const double th = turn[c];
     spp_shift(a, c, f, v.x, v.y, dt, mu);
     a.theta[c] = th;
     if (clear) F[c] = make_double2(0.0, 0.0);
