@@ -98,10 +98,12 @@ static inline bool thread_form_ok(const VoroArgs &a)
     return !a.Ffix && a.tension_mode == 0 && a.K == VG && (reinterpret_cast<uintptr_t>(a.nbr) & 15) == 0;
 }
 
-// Raw calls (no tuner) take it from this many cells on; below, its longer chain per cell shows. us per
-// call of cg_voronoi_forces with its clearing of F, 8-lane / thread form: N = 16384 15.9 / 21.9,
-// 32768 21.7 / 17.5, 65536 20.1 / 19.0, 100003 26.7 / 25.2, 200000 44.3 / 35.7.
-constexpr int RAW_THREAD_CELLS = 148 * 192;
+// Raw calls (no tuner) take it from this many cells on, where the 8-lane form starts its third wave; below,
+// its longer chain per cell shows. us per call of cg_voronoi_forces with its clearing of F, in a captured
+// graph, 8-lane / thread form: N = 28500 8.9 / 10.5, 36000 9.8 / 11.0, 38000 11.9 / 11.1, 50000 13.3 / 12.7,
+// 70000 16.2 / 15.0, 94000 20.8 / 17.2, 100003 21.8 / 21.3 (the thread form's second wave), 120000 25.8 /
+// 22.5, 250000 48.6 / 35.4.
+constexpr int RAW_THREAD_CELLS = 148 * 256;
 
 template <typename R, bool SCATTER, bool TEST>
 static inline void launch_groups(const VoroArgs &a, int N, cudaStream_t st, int shape = 0)
