@@ -212,7 +212,7 @@ static bool persist_vm_ok(const cg_system *s, bool fire)
 
 static int persist_vm_args(cg_system *s, cg::PersistVmArgs &p)
 {
-    if (!s->persist_bar) CG_TRY(dalloc(s, &s->persist_bar, 1));
+    if (!s->persist_bar) CG_TRY(dalloc(s, &s->persist_bar, 2));
     memset(&p, 0, sizeof(p));
     p.a = vm_args(s);
     p.bar = s->persist_bar;
@@ -232,10 +232,7 @@ static int enqueue_vm_persistent(cg_system *s, int kind, int n, double dt, doubl
     p.dt = dt;
     p.mu = mu;
     p.T = T;
-    if (p.a.Ffix)
-        CG_CUDA(cudaMemsetAsync(p.a.Ffix, 0, 2 * FIXF * sizeof(unsigned long long) * s->Nv, s->stream));
-    else
-        CG_CUDA(cudaMemsetAsync(s->F, 0, sizeof(double2) * s->Nv, s->stream));
+    CG_TRY(persist_clear(s, p.a.Ffix));
     void *args[] = {&p};
     return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_vm_steps, args, cg::PVM_SMEM);
 }
@@ -245,6 +242,7 @@ static int enqueue_fire_vm(cg_system *s, int n, cg::FireArgs f)
 {
     cg::PersistVmArgs p;
     CG_TRY(persist_vm_args(s, p));
+    CG_TRY(persist_clear(s, nullptr, false));
     p.steps = n;
     void *args[] = {&p, &f};
     return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_fire_vm, args, cg::PVM_SMEM);
