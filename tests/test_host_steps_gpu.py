@@ -1,8 +1,6 @@
-"""Host-driven steps overlap their copies: the noise of the next step is copied in beside the step that runs,
-so a host step takes no longer than one whose normals are drawn (0.97 of it, reading them being cheaper;
-1.11 where the clearing of the force sums waits behind the copy). The bound is halfway."""
+"""Host-driven steps clear their force sums in a kernel of their own (a memset would wait for the copy of the
+next step's noise that runs beside the step): two launches per step and the clearing one."""
 import ctypes as C
-import time
 
 import numpy as np
 import pytest
@@ -12,13 +10,13 @@ from helpers import jittered_lattice
 pytestmark = pytest.mark.gpu
 
 
-def test_copies_overlap_steps(cglib):
+@pytest.mark.parametrize("nx,ny,kernels", [(20, 15, 2), (300, 300, 3)])  # one launch, two launches
+def test_kernels_of_a_host_step(cglib, nx, ny, kernels):
     import torch
     import cellgpu_b200 as cg
 
-    pos, box = jittered_lattice(300, 300, 0.3, 2)
-    n, steps = len(pos), 40
-    pos = pos[np.random.default_rng(1).permutation(n)]
+    pos, box = jittered_lattice(nx, ny, 0.2, 2)
+    n, steps = len(pos), 5
     b = cg.VoronoiBatch([n], [box])
     b.set_positions(pos)
     b.set_directors(np.zeros(n))
@@ -26,16 +24,10 @@ def test_copies_overlap_steps(cglib):
     b.set_preferences(np.tile([1.0, 3.8], (n, 1)))
     b.triangulate()
     noise = torch.from_numpy(np.random.default_rng(0).standard_normal((steps, n))).pin_memory()
+    before = cglib.cg_kernels_launched(b.handle)
+    for t in range(steps):
+        assert cglib.cg_spp_enqueue_host(b.handle, noise[t].data_ptr(), 0.01, 1.0, None) == 0
     done, halted = C.c_int(0), C.c_int(0)
-
-    def timed(step):
-        t0 = time.perf_counter()
-        for t in range(steps):
-            assert step(t) == 0
-        assert cglib.cg_poll(b.handle, C.byref(done), C.byref(halted), 1) == 0
-        return time.perf_counter() - t0
-
-    host = lambda t: cglib.cg_spp_enqueue_host(b.handle, noise[t].data_ptr(), 0.01, 1.0, None)
-    drawn = lambda t: cglib.cg_spp_enqueue(b.handle, 1, 0.01, 1.0)
-    timed(host), timed(drawn)
-    assert min(timed(host) for _ in range(8)) < 1.04 * min(timed(drawn) for _ in range(8))
+    assert cglib.cg_poll(b.handle, C.byref(done), C.byref(halted), 0) == 0
+    assert (done.value, halted.value) == (steps, 0)
+    assert cglib.cg_kernels_launched(b.handle) - before == kernels * steps
