@@ -306,7 +306,7 @@ struct cg_system {
     std::vector<GraphEntry> graphs;
     long long kernels_enqueued = 0;  // kernels of this library launched for this system
     double *noise_buf = nullptr;     // staging for host-supplied noise (one step)
-    double *draw_buf = nullptr;      // next directors of the step (k_spp_turn)
+    double *draw_buf = nullptr;      // device normals of the step, drawn beside the repair rounds
     // deterministic force sums (cg_set_deterministic): fixed-point accumulator, 4 words per cell
     int det = 0;
     unsigned long long *Ffix = nullptr;
@@ -533,7 +533,7 @@ static size_t voronoi_bytes(int N, int K, int n_bins, int n_inst, int precision)
     size_t per_cell = 4 /*cell_inst*/ + 4 /*held*/ + 4 /*undec*/ + 16 * 3 /*pos, motility, APpref*/ + 8 /*theta*/ + real2 /*AP*/ + 16 /*F*/ +
                       4 + 4 * (size_t)K /*nn, nbr*/ + 4 /*mark*/ + 4 * (R_MAX + 1) /*queue*/ + 4 +
                       4 * (size_t)K /*stage*/ + 4 * 2 /*qslot*/ + 16 /*qhint*/ + 4 /*nclaim*/ + 4 * 3 + 16 /*cell list*/ +
-                      8 + 8 /*noise staging, staged integration*/;
+                      8 + 8 /*noise staging, device draw*/;
     return per_cell * (size_t)N + (size_t)std::min(N, OLD_ROWS) * 4 * (K + 1) /*old rows*/ + (size_t)n_bins * 8 +
            (size_t)n_inst * (sizeof(Inst) + 16) + 4096;
 }
@@ -1264,16 +1264,14 @@ static int build_graph(cg_system *s, int n, double dt, double mu, const double *
         cp.conditional.size = 1;
         cudaGraphNode_t cn;
         CG_CUDA(cudaGraphAddNode(&cn, graph, deps.data(), deps.size(), &cp));
-        // the part of the integration that needs no forces: a kernel node beside the WHILE node
+        // device noise: drawn by a kernel node beside the WHILE node, read by k_spp
         cudaGraphNode_t dn = nullptr;
-        double *turn = s->draw_buf;
-        {
-            double dtv = dt;
-            const double *nzv = noise;
-            void *args[] = {&a, &nzv, &dtv, &turn};
+        if (!noise) {
+            double *out = s->draw_buf;
+            void *args[] = {&a, &out};
             cudaKernelNodeParams kp;
             memset(&kp, 0, sizeof(kp));
-            kp.func = (void *)k_spp_turn;
+            kp.func = (void *)k_draw_noise;
             kp.gridDim = dim3(nblk((s->N + 1) / 2, SPP_BLOCK));
             kp.blockDim = dim3(SPP_BLOCK);
             kp.kernelParams = args;
@@ -1286,19 +1284,21 @@ static int build_graph(cg_system *s, int n, double dt, double mu, const double *
         cudaGraph_t gb;
         CG_CUDA(cudaStreamEndCapture(s->body_stream, &gb));
         deps.assign(1, cn);
-        deps.push_back(dn);
+        if (dn) deps.push_back(dn);
         CG_CUDA(cudaStreamBeginCaptureToGraph(s->stream, graph, deps.data(), nullptr, deps.size(), mode));
+        const double *nz = noise ? noise : s->draw_buf;
         finish_forces<R>(s, a, s->stream);
         // the last step's energy readout: inside its integrator with floating-point sums, else a
         // kernel after the step (fixed-point sums)
         const bool fuse_e = energy_node && t == n - 1 && energy_in_spp(s, false);
         if (fuse_e) {
             k_spp_energy<R><<<nblk((s->N + 1) / 2, SPP_BLOCK), SPP_BLOCK, 0, s->stream>>>(
-                a, turn, dt, mu, s->e2e_acc, s->e2e_done, energy_dst);
+                a, nz, dt, mu, s->e2e_acc, s->e2e_done, energy_dst);
             st = capture_deps(s->stream);
             if (st == CG_OK) *energy_node = deps.empty() ? nullptr : deps[0];
         } else {
-            k_spp_shift<<<nblk(s->N, 256), 256, 0, s->stream>>>(a, turn, dt, mu, !a.Ffix && t + 1 < n);
+            k_spp<R><<<nblk((s->N + 1) / 2, SPP_BLOCK), SPP_BLOCK, 0, s->stream>>>(a, nz, dt, mu, 0u,
+                                                                                   !a.Ffix && t + 1 < n);
         }
         k_step_done<<<1, 1, 0, s->stream>>>(s->ctl, 1);
         s->kernels_enqueued += 2;
@@ -1474,13 +1474,13 @@ static int enqueue_energy_graph(cg_system *s, double dt, double mu, const double
             VoroArgs a = sys_args(s);
             double *acc = s->e2e_acc, *d = dst;
             unsigned *done = s->e2e_done;
-            const double *turn = s->draw_buf;
+            const double *nz = noise ? noise : s->draw_buf;
             double dtv = dt, muv = mu;
             const char *unrolled = getenv("CG_GRAPH_UNROLLED");
             cudaKernelNodeParams kp;
             memset(&kp, 0, sizeof(kp));
             void *args_e[] = {&a, &acc, &done, &d};
-            void *args_s[] = {&a, &turn, &dtv, &muv, &acc, &done, &d};
+            void *args_s[] = {&a, &nz, &dtv, &muv, &acc, &done, &d};
             if (energy_in_spp(s, unrolled && unrolled[0] == '1')) {
                 kp.func = (void *)k_spp_energy<R>;
                 kp.gridDim = dim3(nblk((s->N + 1) / 2, SPP_BLOCK));

@@ -2248,43 +2248,18 @@ __global__ void k_fix_forces(VoroArgs a)
     reinterpret_cast<double2 *>(a.F)[i] = make_double2(fix_force_value(w0, w1), fix_force_value(w2, w3));
 }
 
-// What the step's integration can know before its forces: every cell's velocity and its director after
-// the step, from the given normals or the ones drawn for the current step. The velocities are kept in
-// bin_pos, which only the global triangulation uses (never between this kernel and the shift), the
-// directors in turn[N]. The step graph runs this beside the repair rounds, which leave most of the GPU
-// idle, so that the kernel after them (k_spp_shift) only moves the cells: the integration took 9.3 us of
-// a 262144-cell step and 23 us of a 963507-cell one, most of it in sincos and atan2.
-__global__ void k_spp_turn(VoroArgs a, const double *noise, double dt, double *turn)
+// The same normals for every cell of the current step, into out[N]. The step graph runs this
+// beside the repair rounds (which leave most of the GPU idle), so k_spp reads them instead of
+// drawing them on the step's critical path; the values are the ones k_spp would draw. (Velocities and
+// next directors staged there as well made runs of many steps faster but single steps slower, which the
+// graph is left with: 262144 deterministic cells with L2 flushed 115 -> 123 us.)
+__global__ void k_draw_noise(VoroArgs a, double *out)
 {
     const int c0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (c0 >= a.N) return;
-    const bool two = c0 + 1 < a.N;
-    const double2 xi = noise ? make_double2(noise[c0], two ? noise[c0 + 1] : 0.0) : pair_draw(a, c0, (uint32_t)a.ctl->step);
-    double2 w;
-    turn[c0] = spp_turn(a, c0, xi.x, dt, w.x, w.y);
-    a.bin_pos[c0] = w;
-    if (two) {
-        turn[c0 + 1] = spp_turn(a, c0 + 1, xi.y, dt, w.x, w.y);
-        a.bin_pos[c0 + 1] = w;
-    }
-}
-
-// the rest of the integration of cell c; clear: its force sum is zeroed for the next step
-CG_D void spp_staged(const VoroArgs &a, int c, const double *turn, double dt, double mu, int clear)
-{
-    double2 *F = reinterpret_cast<double2 *>(a.F);
-    const double2 f = F[c], v = a.bin_pos[c];
-    const double th = turn[c];
-    spp_shift(a, c, f, v.x, v.y, dt, mu);
-    a.theta[c] = th;
-    if (clear) F[c] = make_double2(0.0, 0.0);
-}
-
-__global__ void __launch_bounds__(256) k_spp_shift(VoroArgs a, const double *turn, double dt, double mu, int clear)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.N || (a.ctl && a.ctl->halt)) return;
-    spp_staged(a, c, turn, dt, mu, clear);
+    const double2 xi = pair_draw(a, c0, (uint32_t)a.ctl->step);
+    out[c0] = xi.x;
+    if (c0 + 1 < a.N) out[c0 + 1] = xi.y;
 }
 
 template <typename R>
@@ -2424,12 +2399,12 @@ __global__ void __launch_bounds__(256) k_energy_to_host(VoroArgs a, double *acc,
 }
 
 // The step's integration with its energy readout (host-energy steps with floating-point force
-// sums): the staged integration (k_spp_shift), two cells per thread, whose energies (of the configuration the forces were
+// sums): k_spp's two cells per thread, whose energies (of the configuration the forces were
 // computed on: A/P are not changed by the move) are summed per block of 256 cells and per instance
 // as k_energy_to_host sums them, the last block storing the totals to the host buffer. One kernel
 // instead of the integrator and a separate readout after the step's epilogue.
 template <typename R>
-__global__ void __launch_bounds__(128) k_spp_energy(VoroArgs a, const double *turn, double dt, double mu, double *acc,
+__global__ void __launch_bounds__(128) k_spp_energy(VoroArgs a, const double *noise, double dt, double mu, double *acc,
                                                     unsigned *done, double *host_out)
 {
     __shared__ double s_part[4];
@@ -2449,8 +2424,11 @@ __global__ void __launch_bounds__(128) k_spp_energy(VoroArgs a, const double *tu
         n1 = a.cell_inst ? a.cell_inst[c0 + 1] : 0;
     }
     if (one && !(ctl && ctl->halt)) {  // a halted step does not move (the host recovers it)
-        spp_staged(a, c0, turn, dt, mu, 0);
-        if (two) spp_staged(a, c0 + 1, turn, dt, mu, 0);
+        double2 xi;
+        if (noise) xi = make_double2(noise[c0], two ? noise[c0 + 1] : 0.0);
+        else xi = pair_draw(a, c0, ctl ? (uint32_t)ctl->step : 0u);
+        spp_cell<R>(a, c0, xi.x, dt, mu, 0);
+        if (two) spp_cell<R>(a, c0 + 1, xi.y, dt, mu, 0);
     }
     const int b0 = 2 * blockIdx.x * blockDim.x, b1 = min(a.N, b0 + 2 * (int)blockDim.x) - 1;
     const int i0 = a.cell_inst ? a.cell_inst[b0] : 0, i1 = a.cell_inst ? a.cell_inst[b1] : 0;
