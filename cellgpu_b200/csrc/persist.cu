@@ -793,6 +793,7 @@ static int persist_args(cg_system *s, int grid, cg::PersistArgs &p)
     if (!s->persist_bar) CG_TRY(dalloc(s, &s->persist_bar, 2));
     memset(&p, 0, sizeof(p));
     p.a = sys_args(s);
+    p.a.old_cap = std::min(s->N, OLD_ROWS);  // commit and check on two warps
     p.bar = s->persist_bar;
     p.absent = s->stall_ns ? 1 : 0;
     p.wait_ns = s->stall_ns ? s->stall_ns : cg::PERSIST_WAIT_NS;

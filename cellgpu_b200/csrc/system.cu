@@ -504,7 +504,6 @@ static VoroArgs sys_args(cg_system *s)
     a.stage_nbr = s->stage_nbr;
     a.old_nn = s->old_nn;
     a.old_nbr = s->old_nbr;
-    a.old_cap = s->old_nbr ? std::min(s->N, OLD_ROWS) : 0;
     a.qslot = s->qslot;
     a.qhint = s->qhint;
     a.nclaim = s->nclaim;
@@ -1086,15 +1085,13 @@ static int grow_rows(cg_system *s)
     CG_CUDA(cudaStreamSynchronize(s->stream));
     for (auto &g : s->graphs) release_graph(g);
     s->graphs.clear();
-    int *nbr2 = nullptr, *stage2 = nullptr, *old2 = nullptr;
-    CG_TRY(dalloc(s, &old2, (size_t)std::min(s->N, OLD_ROWS) * K2));
+    int *nbr2 = nullptr, *stage2 = nullptr;
     CG_TRY(dalloc(s, &nbr2, (size_t)s->N * K2));
     CG_TRY(dalloc(s, &stage2, (size_t)s->N * K2));
     k_widen_rows<<<nblk(s->N, 256), 256, 0, s->stream>>>(s->N, s->K, K2, s->nbr, nbr2);
     CG_TRY(check_launch());
     s->nbr = nbr2;  // (the old blocks stay in the arena until the system is destroyed)
     s->stage_nbr = stage2;
-    s->old_nbr = old2;
     if (s->sort_tmp)
         CG_TRY(dalloc(s, (char **)&s->sort_tmp, (size_t)s->N * std::max<size_t>(16, sizeof(int) * (size_t)(K2 + 1))));
     s->K = K2;

@@ -1508,7 +1508,9 @@ CG_D const int *future_row(const VoroArgs &a, int x, int round, int nq, const in
 // Commit and check queue slots base and base + 1 of `round` (whole warp: 16 lanes per slot, the
 // warp's four group tiles in wt). The two halves, commit (forces, exact test, row replacement) and
 // check (the partners' rows), are chains of about equal length that share only the rows; where the
-// old rows are kept (old_cap) two warps take one each (PART 1 and 2; PART 0: both in turn).
+// old rows are kept (old_cap: the cooperative forms) two warps take one each (PART 1 and 2; PART 0: both in
+// turn). As kernels of their own the halves gained 1 us of a warm step and lost 4 to 8 us with cold
+// caches (262144 cells: deterministic 117 -> 121, mixed 104 -> 112).
 constexpr int CC_BOTH = 0, CC_COMMIT = 1, CC_CHECK = 2;
 
 template <typename R, bool FORCES, int NS, int PART>
@@ -1671,16 +1673,8 @@ __global__ void __launch_bounds__(WPB * 32) k_commit_check(VoroArgs a, unsigned 
         const int e_next = ctl->epoch + round + 1;  // claim epoch of the next round
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         const int step = gridDim.x * WPB * (GPW / 2);
-        const bool split = nq <= a.old_cap;  // an even warp commits and the next one checks the same slots
-        const int first = split ? (blockIdx.x * WPB + w) / 2 : blockIdx.x * WPB + w;
-        for (int base = first * (GPW / 2); base < nq; base += split ? step / 2 : step) {  // warp-uniform
-            if (!split)
-                cc_pair<R, FORCES, NS, CC_BOTH>(a, ctl, round, nq, queue, e_next, base, tile + w * GPW, lane);
-            else if ((w & 1) == 0)
-                cc_pair<R, FORCES, NS, CC_COMMIT>(a, ctl, round, nq, queue, e_next, base, tile + w * GPW, lane);
-            else
-                cc_pair<R, FORCES, NS, CC_CHECK>(a, ctl, round, nq, queue, e_next, base, tile + w * GPW, lane);
-        }
+        for (int base = (blockIdx.x * WPB + w) * (GPW / 2); base < nq; base += step)  // warp-uniform
+            cc_pair<R, FORCES, NS, CC_BOTH>(a, ctl, round, nq, queue, e_next, base, tile + w * GPW, lane);
     }
     // the last block to finish ends the round (threadfence reduction: every block's claims are
     // visible before its count is)
