@@ -624,11 +624,9 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_fire_voro(PersistArgs p
 
 }  // namespace cg
 
-// Largest systems that step in one cooperative launch: runs of several steps (with the thread-per-cell
-// force pass / with the 8-lane one), single steps (the host steps, where each launch brings its own
-// clearing of the sums and the host's share of a launch) and single steps in the deterministic mode
-// (64 bytes of sums per cell and a readout kernel). Larger systems take two launches per step, the
-// force pass as a kernel of its own occupancy and k_voro_tail.
+// Largest systems that step in one cooperative launch, with the thread-per-cell force pass / with the
+// 8-lane one. Larger systems take two launches per step, the force pass as a kernel of its own occupancy
+// and k_voro_tail.
 // us per step of a relaxed tissue, one launch / two per step / the graph:
 //               FP64                  deterministic         mixed
 //   N = 300      8.6 /  -   / 24.1     8.7 /  -   / 22.1     8.5 /  -   / 20.6
@@ -637,22 +635,26 @@ __global__ void __launch_bounds__(PERSIST_WPB * 32, 1) k_fire_voro(PersistArgs p
 //   N = 65536   36.3 / 37.3 / 47      46.6 / 43.3 / 55      44.1 / 39.2 / 51
 //   N = 100000  49.2 / 45.6 / 58      63.5 / 53.6 / 64      57.1 / 47.5 / 58
 //   N = 262144  81.1 / 70.0 / 75.0      -  / 96.6 / 101       -  / 81.3 / 87.4
-// host steps: N = 300 19.7 / - / 29.4 and 24.3 / - / 27.7 (deterministic), 8192 31.7 / - / 38.4 and
-// 37.0 / - / 36.3, 65536 57.4 / 58.2 / 59.0
 constexpr int PERSIST_MAX_THREAD = 81920, PERSIST_MAX_CELLS = 30000;
-constexpr int PERSIST_MAX_SINGLE = 65536, PERSIST_MAX_SINGLE_FIX = 1024;
-// Single steps with fixed-point sums or in mixed precision above this many cells go through the step
-// graph: its integration runs beside the repair and at full occupancy, and these modes convert sums or
-// hold the force pass for longer. us per host step / single step / single step with L2 flushed, two
-// launches against the graph:
-//                deterministic                          mixed
-//   N =  66560    62 /  46 /  63    59 /  45 /  68       50 /  40 /  60    54 /  43 /  68
-//   N = 100000    77 /  58 /  76    71 /  59 /  82       65 /  51 /  70    62 /  50 /  72
-//   N = 180000   100 /  84 / 102    89 /  79 /  98       83 /  71 /  88    78 /  70 /  88
-//   N = 262144   125 / 107 / 125   110 / 101 / 121       96 /  87 / 106    95 /  86 / 102
-// FP64 with atomic sums: two launches at every size (100000 64 / 47 / 69 against 61 / 48 / 74, 262144 82 /
-// 68 / 86 against 82 / 70 / 90).
-constexpr int PERSIST_MAX_TWO_SINGLE = 90000;
+// Single steps bring their own clearing of the sums and the host's share of a launch. us per host step (noise
+// in, energy out) / step with drawn normals, a tissue in random order, one launch against two; the step
+// graph before there were such forms:
+//   FP64     N = 16000  27 / 25   34 / 26    40 / 29       tension  N =  9000  27 / 22   28 / 23    35 / 25
+//            N = 31000  34 / 28   36 / 28    44 / 32                N = 16000  32 / 26   32 / 25    41 / 28
+//            N = 60000  41 / 35   45 / 35    54 / 37                N = 31000  43 / 35   39 / 31    50 / 35
+//            N = 90000    -       49 / 40    62 / 44                N = 60000  64 / 50   52 / 44    61 / 49
+//   mixed    N = 16000  27 / 25   28 / 23    34 / 25       deterministic 4000  28 / 20   28 / 21    32 / 25
+//            N = 31000  38 / 32   35 / 27    42 / 30                N = 31000     -      42 / 32    47 / 33
+//            N = 60000  52 / 45   46 / 36    55 / 41                N = 90000     -      63 / 50    72 / 56
+constexpr int PERSIST_MAX_SINGLE = 65536;        // FP64, whose force pass has the thread-per-cell form
+constexpr int PERSIST_MAX_SINGLE_CELLS = 16384;  // the 8-lane form
+constexpr int PERSIST_MAX_SINGLE_FIX = 1024;     // fixed-point sums: 64 bytes per cell, a readout kernel
+// Single deterministic steps above this size go through the step graph, which converts the sums and
+// integrates at full occupancy. us per host step / drawn step / the same with L2 flushed, two launches
+// against the graph: 100000 cells 70 / 58 / 77 and 73 / 62 / 80, 131072 78 / 66 / 85 and 78 / 69 / 88,
+// 180000 91 / 82 / 100 and 90 / 83 / 96, 262144 119 / 107 / 129 and 111 / 102 / 117. (Mixed precision takes two
+// launches: 262144 94 / 87 / 104 and 99 / 90 / 106.)
+constexpr int PERSIST_MAX_TWO_FIX = 131072;
 
 template <typename R, int FIX>
 static const void *persist_kernel() { return (const void *)cg::k_voro_steps<R, FIX>; }
@@ -712,11 +714,13 @@ static StepForm step_form(const cg_system *s, int n)
 {
     if (!persist_any(s)) return STEP_GRAPH;
     if (n == 1) {
-        const bool small = s->N <= (s->det ? PERSIST_MAX_SINGLE_FIX : PERSIST_MAX_SINGLE);
+        const bool small = s->N <= (s->det                  ? PERSIST_MAX_SINGLE_FIX
+                                    : persist_thread_ok(s) ? PERSIST_MAX_SINGLE
+                                                           : PERSIST_MAX_SINGLE_CELLS);
         const int others = n_busy[s->device & 63].load() - (s->busy ? 1 : 0);
         if (others > 0) return small && others == 1 && 2 * persist_grid(s) <= s->sms ? STEP_ONE : STEP_GRAPH;
         if (small) return STEP_ONE;
-        return s->N > PERSIST_MAX_TWO_SINGLE && (s->det || s->precision != CG_FP64) ? STEP_GRAPH : STEP_TWO;
+        return s->det && s->N > PERSIST_MAX_TWO_FIX ? STEP_GRAPH : STEP_TWO;
     }
     return s->N <= (persist_thread_ok(s) ? PERSIST_MAX_THREAD : PERSIST_MAX_CELLS) ? STEP_ONE : STEP_TWO;
 }

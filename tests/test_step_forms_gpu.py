@@ -71,7 +71,9 @@ def test_runs(cglib, torch, monkeypatch, sizes, opts, drawn):
 # one launch, two launches, the step graph, two launches and an integrator of its own
 @pytest.mark.parametrize("sizes,opts", [([(256, 256)], ""), ([(260, 256)], ""), ([(450, 440)], ""), ([(460, 440)], ""),
                                         ([(300, 298)], "mixed"), ([(310, 298)], "mixed"),
-                                        ([(300, 298)], "deterministic"), ([(310, 298)], "deterministic")])
+                                        ([(300, 298)], "deterministic"), ([(310, 298)], "deterministic"),
+                                        ([(128, 128)], "mixed"), ([(129, 128)], "mixed"),
+                                        ([(362, 362)], "deterministic"), ([(363, 362)], "deterministic")])
 @pytest.mark.parametrize("drawn", [True, False])
 def test_single_steps(cglib, oracle, torch, monkeypatch, sizes, opts, drawn):
     b, n, rng, pref = make(sizes, opts)
