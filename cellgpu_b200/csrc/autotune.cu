@@ -5,8 +5,10 @@
 // and at least 16 blocks per SM, or 4 warps with at least 8, or one thread per cell) and the
 // cell-list bin side of the global triangulation
 // (0.8, 1.0 or 1.25 mean cell spacings; the bin arrays allocated at creation hold all three).
+// The force shape is read by steps of two launches, the step graph, FIRE graphs and single force passes;
+// steps in one launch choose theirs by the cells per block (persist.cu).
 // cg_autotune_repair times the grids of the repair round's two launches on real SPP steps, which
-// are the only way to get a representative repair load. The repair queues hold every cell of the
+// are the only way to get a representative repair load; graphs read them, and the steps run through one. The repair queues hold every cell of the
 // system per round, so they cannot overflow and have no capacity to tune; the local star's
 // candidate capacity is a compile-time shared-memory size. Cached step graphs are dropped so the
 // next run captures the chosen shapes.

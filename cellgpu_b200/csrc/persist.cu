@@ -681,7 +681,12 @@ constexpr int PERSIST_CLUSTER = 16;
 constexpr int PERSIST_THREAD_CELLS = 192;
 
 // One block per SM at most, and no more blocks than the cells fill. Calls that run at the same time on
-// other systems take their share of the SMs: grids that fill the GPU would take turns.
+// other systems take their share of the SMs: grids that fill the GPU would take turns. us per step or
+// iteration of all of M systems in M threads, full grids / shared ones / graphs:
+//   FIRE 16384 cells  M = 2  42 / 31 / 51    4   83 / 44 /  72    8  163 /  58 / 122
+//   FIRE 65536        M = 2  55 / 48 / 67    4  108 / 90 /  98    8  219 / 151 / 196
+//   SPP  16384        M = 2  38 / 24 / 52    4   74 / 31 /  71    8  147 /  46 / 123
+//   SPP  65536        M = 2  58 / 48 / 69    4  116 / 82 /  99    8  233 / 147 / 194
 static int persist_grid(const cg_system *s)
 {
     const int share = s->in_run ? std::max(1, s->sms / std::max(1, n_running[s->device & 63].load())) : s->sms;
@@ -694,8 +699,8 @@ static int persist_grid(const cg_system *s)
 // 81.5 -> 81.1); at 180000 75.8 -> 73.8, 59.1 -> 60.4, 73.4 -> 73.5.
 constexpr int SPLIT_MOVE_CELLS = 300000, SPLIT_MOVE_SINGLE = 200000;
 
-// Whether steps can run without the step graph: the device takes the launches, 32-slot rows need the wide forms of the repair, and the
-// profiling form unrolls graphs.
+// Whether steps can run without the step graph: the device takes the launches, 32-slot rows need the wide
+// forms of the repair, and the profiling form unrolls graphs.
 static bool persist_any(const cg_system *s)
 {
     const char *u = getenv("CG_GRAPH_UNROLLED");

@@ -676,7 +676,7 @@ extern "C" int cg_device_memory(size_t *free_bytes, size_t *total_bytes)
 extern "C" int cg_set_stream(cg_system *s, cudaStream_t stream)
 {
     if (!s) return set_err(CG_ERR_ARG, "null system");
-    CG_CUDA(cudaStreamSynchronize(s->stream));
+    CG_TRY(cg_synchronize(s));
     s->stream = stream ? stream : s->own_stream;
     return CG_OK;
 }

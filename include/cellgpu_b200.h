@@ -212,7 +212,9 @@ int cg_set_instance_seeds(cg_system *sys, const uint64_t *seeds);
 int cg_set_deterministic(cg_system *sys, int on);
 int cg_get_deterministic(cg_system *sys);
 int cg_spp_run(cg_system *sys, int n_steps, double dt, double mu, const double *noise_dev);
-/* Enqueue n_steps RNG-driven SPP steps (one CUDA graph replay) with no host synchronisation.
+/* Enqueue n_steps RNG-driven SPP steps (cooperative launches or a CUDA graph) with no host synchronisation.
+ * Steps and iterations of several systems share the GPU by how many systems have work enqueued that no
+ * call of this library has waited for yet (cg_synchronize, cg_poll or any call that reads or sets state).
  * A step that cannot finish on the device (a global rebuild is needed) sets a sticky halt flag and
  * the remaining enqueued steps do nothing; cg_poll reports completed steps and recovers. */
 int cg_spp_enqueue(cg_system *sys, int n_steps, double dt, double mu);
@@ -371,7 +373,9 @@ int cg_autotune(cg_system *sys, double *times_ms, int *choice);
 
 /* Repair-launch autotuner (no counterpart in the reference): times the grids of the local repair
  * round's two launches (k_star_local: 148 x 5 or 148 x 2 blocks; k_commit_check: 148 x 4, 8 or 16)
- * on real SPP steps with device noise, `steps` steps twice per pair, and keeps the fastest. The
+ * on real SPP steps with device noise, `steps` steps twice per pair, and keeps the fastest. The grids
+ * are those of the step graph (wide rows, large deterministic single steps, single steps beside other
+ * systems') and of FIRE graphs; the cooperative forms of a step have none to tune. The
  * system ADVANCES by 12 x steps steps (run it in place of equilibration steps). The repair queues
  * hold every cell per round and cannot overflow, so they have no capacity to tune. times_ms (6
  * values, ms per step, star grid major) and choice (the two grids) may be NULL. Voronoi systems only
