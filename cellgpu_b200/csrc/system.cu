@@ -714,8 +714,54 @@ static int h2d(cg_system *s, void *dst, const void *src, size_t b)
     return CG_OK;
 }
 
+// Small read-backs go through a page-locked page, one copy and one wait. Pages are made as concurrent
+// calls need them and kept for the next call, up to KEEP_PAGES.
+constexpr size_t PAGE_BYTES = 4096, KEEP_PAGES = 32;
+static std::mutex page_mutex;
+static std::vector<void *> free_pages;
+
+struct HostPage {
+    void *p = nullptr;
+    HostPage()
+    {
+        {
+            std::lock_guard<std::mutex> lock(page_mutex);
+            if (!free_pages.empty()) {
+                p = free_pages.back();
+                free_pages.pop_back();
+                return;
+            }
+        }
+        if (cudaHostAlloc(&p, PAGE_BYTES, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~HostPage()
+    {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lock(page_mutex);
+            if (free_pages.size() < KEEP_PAGES) {
+                free_pages.push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+};
+
 static int d2h(cg_system *s, void *dst, const void *src, size_t b)
 {
+    if (b <= PAGE_BYTES) {
+        HostPage page;
+        if (page.p) {
+            CG_CUDA(cudaMemcpyAsync(page.p, src, b, cudaMemcpyDeviceToHost, s->stream));
+            CG_TRY(cg_synchronize(s));
+            memcpy(dst, page.p, b);
+            return CG_OK;
+        }
+    }
     CG_TRY(settle(s));
     CG_CUDA(cudaMemcpyAsync(dst, src, b, cudaMemcpyDeviceToHost, s->stream));
     CG_CUDA(cudaStreamSynchronize(s->stream));
