@@ -681,7 +681,7 @@ constexpr int PERSIST_CLUSTER = 16;
 constexpr int PERSIST_THREAD_CELLS = 192;
 
 // One block per SM at most, and no more blocks than the cells fill. Calls that run at the same time on
-// other systems take their share of the SMs: grids that fill the GPU would take turns. us per step or
+// other streams take their share of the SMs: grids that fill the GPU would take turns. us per step or
 // iteration of all of M systems in M threads, full grids / shared ones / graphs:
 //   FIRE 16384 cells  M = 2  42 / 31 / 51    4   83 / 44 /  72    8  163 /  58 / 122
 //   FIRE 65536        M = 2  55 / 48 / 67    4  108 / 90 /  98    8  219 / 151 / 196
@@ -689,7 +689,7 @@ constexpr int PERSIST_THREAD_CELLS = 192;
 //   SPP  65536        M = 2  58 / 48 / 69    4  116 / 82 /  99    8  233 / 147 / 194
 static int persist_grid(const cg_system *s)
 {
-    const int share = s->in_run ? std::max(1, s->sms / std::max(1, n_running[s->device & 63].load())) : s->sms;
+    const int share = s->in_run ? std::max(1, s->sms / (1 + running_streams.others(s))) : s->sms;
     return std::max(1, std::min(share, nblk(s->N, cg::PERSIST_WPB * GPW)));
 }
 
@@ -709,7 +709,7 @@ static bool persist_any(const cg_system *s)
 
 enum StepForm { STEP_GRAPH, STEP_ONE, STEP_TWO };  // the step graph, one launch, two launches per step
 
-// The form that n steps take. Single steps beside other systems' (host-driven ones on several streams) go
+// The form that n steps take. Single steps beside those of other streams (host-driven systems) go
 // through the step graph, whose kernels overlap with theirs; two small systems also fit side by side.
 // us per round of single steps of M systems, one launch / graph:
 //   300 cells    M = 2  21 / 29    4  40 / 30    8   66 / 37
@@ -722,7 +722,7 @@ static StepForm step_form(const cg_system *s, int n)
         const bool small = s->N <= (s->det                  ? PERSIST_MAX_SINGLE_FIX
                                     : persist_thread_ok(s) ? PERSIST_MAX_SINGLE
                                                            : PERSIST_MAX_SINGLE_CELLS);
-        const int others = n_busy[s->device & 63].load() - (s->busy ? 1 : 0);
+        const int others = busy_streams.others(s);
         if (others > 0) return small && others == 1 && 2 * persist_grid(s) <= s->sms ? STEP_ONE : STEP_GRAPH;
         if (small) return STEP_ONE;
         return s->det && s->N > PERSIST_MAX_TWO_FIX ? STEP_GRAPH : STEP_TWO;

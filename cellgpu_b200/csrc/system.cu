@@ -1,11 +1,11 @@
 // cellgpu_b200 -- host side of the C ABI: kernel callers on caller memory, and the device-resident
 // batched system (cg_system). Built as one translation unit with the kernel files.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -422,22 +422,40 @@ static int dalloc(cg_system *s, T **p, size_t count)
     return CG_OK;
 }
 
-// Per device, the systems with steps enqueued and not yet waited for, and those inside a call that runs
-// steps and waits for them. They share the GPU: the launch forms that hold whole SMs (persist.cu) look
-// at these counts, which change no result.
-static std::atomic<int> n_busy[64], n_running[64];
+// The streams with steps enqueued and not yet waited for, and those inside a call that runs steps and
+// waits for them, with the number of their systems. Work of different streams shares the GPU (systems
+// on one stream follow one another anyway): the launch forms that hold whole SMs (persist.cu) ask how
+// many others there are, which changes no result. (Never destroyed: other threads may outlive exit.)
+struct StreamUse {
+    std::mutex m;
+    std::map<std::pair<int, cudaStream_t>, int> n;  // by device and stream
+    void add(const cg_system *s, int d)
+    {
+        std::lock_guard<std::mutex> lock(m);
+        const auto it = n.emplace(std::make_pair(s->device, s->stream), 0).first;
+        if ((it->second += d) == 0) n.erase(it);
+    }
+    int others(const cg_system *s)
+    {
+        std::lock_guard<std::mutex> lock(m);
+        int k = 0;
+        for (const auto &e : n) k += e.first.first == s->device && e.first.second != s->stream;
+        return k;
+    }
+};
+static StreamUse &busy_streams = *new StreamUse, &running_streams = *new StreamUse;
 
-static void mark(bool &flag, std::atomic<int> *count, const cg_system *s, bool on)
+static void mark(bool &flag, StreamUse &use, const cg_system *s, bool on)
 {
     if (flag == on) return;
     flag = on;
-    count[s->device & 63] += on ? 1 : -1;
+    use.add(s, on ? 1 : -1);
 }
 
 struct RunScope {
     cg_system *s;
-    explicit RunScope(cg_system *sys) : s(sys) { mark(s->in_run, n_running, s, true); }
-    ~RunScope() { mark(s->in_run, n_running, s, false); }
+    explicit RunScope(cg_system *sys) : s(sys) { mark(s->in_run, running_streams, s, true); }
+    ~RunScope() { mark(s->in_run, running_streams, s, false); }
 };
 
 // streams of a new system (before any allocation)
@@ -455,7 +473,7 @@ static int sys_streams(cg_system *s)
 static void sys_release(cg_system *s)
 {
     if (s->stream) cudaStreamSynchronize(s->stream);
-    mark(s->busy, n_busy, s, false);
+    mark(s->busy, busy_streams, s, false);
     for (auto &g : s->graphs) release_graph(g);
     s->graphs.clear();
     cudaStream_t fs = s->own_stream;
@@ -684,7 +702,7 @@ extern "C" int cg_set_stream(cg_system *s, cudaStream_t stream)
 extern "C" cudaStream_t cg_get_stream(cg_system *s) { return s ? s->stream : nullptr; }
 
 // steps or iterations of the system are enqueued
-static void enqueued(cg_system *s) { mark(s->busy, n_busy, s, true); }
+static void enqueued(cg_system *s) { mark(s->busy, busy_streams, s, true); }
 
 // Wait for them. A copy to or from pageable memory behind a launch of hundreds of steps would wait for
 // it inside the driver, with a lock that keeps every other thread from launching: four threads, each
@@ -694,7 +712,7 @@ static int settle(cg_system *s)
 {
     if (!s->busy) return CG_OK;
     CG_CUDA(cudaStreamSynchronize(s->stream));
-    mark(s->busy, n_busy, s, false);
+    mark(s->busy, busy_streams, s, false);
     return CG_OK;
 }
 
@@ -702,7 +720,7 @@ extern "C" int cg_synchronize(cg_system *s)
 {
     if (!s) return set_err(CG_ERR_ARG, "null system");
     CG_CUDA(cudaStreamSynchronize(s->stream));
-    mark(s->busy, n_busy, s, false);
+    mark(s->busy, busy_streams, s, false);
     return CG_OK;
 }
 
@@ -717,8 +735,8 @@ static int h2d(cg_system *s, void *dst, const void *src, size_t b)
 // Small read-backs go through a page-locked page, one copy and one wait. Pages are made as concurrent
 // calls need them and kept for the next call, up to KEEP_PAGES.
 constexpr size_t PAGE_BYTES = 4096, KEEP_PAGES = 32;
-static std::mutex page_mutex;
-static std::vector<void *> free_pages;
+static std::mutex &page_mutex = *new std::mutex;
+static std::vector<void *> &free_pages = *new std::vector<void *>;
 
 struct HostPage {
     void *p = nullptr;
@@ -756,6 +774,9 @@ static int d2h(cg_system *s, void *dst, const void *src, size_t b)
     if (b <= PAGE_BYTES) {
         HostPage page;
         if (page.p) {
+            // beside other streams the copy is not queued behind the steps: streams beyond the device's
+            // connections share one, and theirs would wait for it (eight 300-cell FIRE runs 20 against 12 us)
+            if (s->busy && busy_streams.others(s) > 0) CG_TRY(settle(s));
             CG_CUDA(cudaMemcpyAsync(page.p, src, b, cudaMemcpyDeviceToHost, s->stream));
             CG_TRY(cg_synchronize(s));
             memcpy(dst, page.p, b);

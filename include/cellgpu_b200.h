@@ -213,8 +213,9 @@ int cg_set_deterministic(cg_system *sys, int on);
 int cg_get_deterministic(cg_system *sys);
 int cg_spp_run(cg_system *sys, int n_steps, double dt, double mu, const double *noise_dev);
 /* Enqueue n_steps RNG-driven SPP steps (cooperative launches or a CUDA graph) with no host synchronisation.
- * Steps and iterations of several systems share the GPU by how many systems have work enqueued that no
- * call of this library has waited for yet (cg_synchronize, cg_poll or any call that reads or sets state).
+ * Steps and iterations of systems on several streams share the GPU by how many streams have work enqueued
+ * that no call of this library has waited for yet (cg_synchronize, cg_poll or any call that reads or sets
+ * state).
  * A step that cannot finish on the device (a global rebuild is needed) sets a sticky halt flag and
  * the remaining enqueued steps do nothing; cg_poll reports completed steps and recovers. */
 int cg_spp_enqueue(cg_system *sys, int n_steps, double dt, double mu);
