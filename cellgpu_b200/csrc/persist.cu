@@ -747,12 +747,18 @@ static int persist_refused(cg_system *s)
     return PERSIST_REFUSED;
 }
 
+// Whether a launch of this grid is one cluster (whose hardware barrier has no limit to run out).
+static bool persist_cluster(const cg_system *s, int grid)
+{
+    return grid <= PERSIST_CLUSTER && !s->stall_ns && !s->inject_refusal;
+}
+
 // A cooperative launch, or one cluster where the grid is small and a GPC has room for it (*cluster, an
 // argument of the kernel, is set accordingly).
 static int persist_launch(cg_system *s, int grid, int *cluster, const void *kernel, void **args, size_t smem)
 {
+    *cluster = persist_cluster(s, grid);
     if (s->inject_refusal) grid = 4 * s->sms;  // (a block takes an SM)
-    *cluster = grid <= PERSIST_CLUSTER && !s->stall_ns;  // (the hardware barrier has no limit to run out)
     CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -773,6 +779,7 @@ static int persist_launch(cg_system *s, int grid, int *cluster, const void *kern
         if (launch_refused(e)) {
             cudaGetLastError();
             *cluster = 0;
+            CG_CUDA(cudaMemsetAsync(s->persist_bar, 0, 2 * sizeof(unsigned), s->stream));
         }
     }
     if (!*cluster) {
@@ -787,12 +794,19 @@ static int persist_launch(cg_system *s, int grid, int *cluster, const void *kern
     return CG_OK;
 }
 
-// before a launch: force sums (fixed-point ones where fix) and barrier counters at zero
-static int persist_clear(cg_system *s, const unsigned long long *fix, bool sums = true)
+// Before a launch: force sums (fixed-point ones where fix) and barrier counters at zero. One cluster needs no
+// counters, and its few sums are cleared sooner by a memset (400 cells in mixed precision 21.5 against 23.3
+// us per host step, 100 cells 23.7 against 24.8).
+static int persist_clear(cg_system *s, int grid, const unsigned long long *fix, bool sums = true)
 {
     const long long n = sums ? (long long)ndof(s) * (fix ? 2 * FIXF / 2 : 1) : 0;
+    void *p = fix ? (void *)s->Ffix : (void *)s->F;
+    if (persist_cluster(s, grid)) {
+        if (n) CG_CUDA(cudaMemsetAsync(p, 0, sizeof(ulonglong2) * n, s->stream));
+        return CG_OK;
+    }
     k_persist_clear<<<std::max(1, std::min(8 * s->sms, nblk((int)std::min(n, 1ll << 30), 256))), 256, 0, s->stream>>>(
-        reinterpret_cast<ulonglong2 *>(fix ? (void *)s->Ffix : (void *)s->F), n, s->persist_bar);
+        reinterpret_cast<ulonglong2 *>(p), n, s->persist_bar);
     s->kernels_enqueued += 1;
     return check_launch();
 }
@@ -823,7 +837,7 @@ static int enqueue_fire_persistent(cg_system *s, int n, cg::FireArgs f)
     cg::PersistArgs p;
     const int grid = persist_grid(s);
     CG_TRY(persist_args(s, grid, p));
-    CG_TRY(persist_clear(s, nullptr, false));
+    CG_TRY(persist_clear(s, grid, nullptr, false));
     p.steps = n;
     void *args[] = {&p, &f};
     return persist_launch(s, grid, &p.cluster, (const void *)cg::k_fire_voro, args, cg::PERSIST_SMEM);
@@ -881,7 +895,7 @@ static int enqueue_persistent(cg_system *s, StepForm form, int n, double dt, dou
         p.host_out = energy_dst;
     }
     const void *k = p.a.Ffix ? persist_kernel<R, 1>() : persist_kernel<R, 0>();
-    CG_TRY(persist_clear(s, p.a.Ffix));
+    CG_TRY(persist_clear(s, form == STEP_ONE ? grid : s->sms, p.a.Ffix));
     if (form == STEP_ONE) {
         void *args[] = {&p};
         const int st = persist_launch(s, grid, &p.cluster, k, args, cg::PERSIST_SMEM);

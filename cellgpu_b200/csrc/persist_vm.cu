@@ -232,9 +232,10 @@ static int enqueue_vm_persistent(cg_system *s, int kind, int n, double dt, doubl
     p.dt = dt;
     p.mu = mu;
     p.T = T;
-    CG_TRY(persist_clear(s, p.a.Ffix));
+    const int grid = persist_grid(s);
+    CG_TRY(persist_clear(s, grid, p.a.Ffix));
     void *args[] = {&p};
-    return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_vm_steps, args, cg::PVM_SMEM);
+    return persist_launch(s, grid, &p.cluster, (const void *)cg::k_vm_steps, args, cg::PVM_SMEM);
 }
 
 // up to n FIRE iterations, enqueued, or PERSIST_REFUSED (the FIRE state is set up and F holds the current forces)
@@ -242,8 +243,9 @@ static int enqueue_fire_vm(cg_system *s, int n, cg::FireArgs f)
 {
     cg::PersistVmArgs p;
     CG_TRY(persist_vm_args(s, p));
-    CG_TRY(persist_clear(s, nullptr, false));
+    const int grid = persist_grid(s);
+    CG_TRY(persist_clear(s, grid, nullptr, false));
     p.steps = n;
     void *args[] = {&p, &f};
-    return persist_launch(s, persist_grid(s), &p.cluster, (const void *)cg::k_fire_vm, args, cg::PVM_SMEM);
+    return persist_launch(s, grid, &p.cluster, (const void *)cg::k_fire_vm, args, cg::PVM_SMEM);
 }

@@ -1,5 +1,5 @@
-"""Host-driven steps clear their force sums in a kernel of their own (a memset would wait for the copy of the
-next step's noise that runs beside the step): two launches per step and the clearing one."""
+"""Host-driven steps of large systems clear their force sums in a kernel of their own (a memset would wait for
+the copy of the next step's noise that runs beside the step), small ones, one cluster, by a memset."""
 import ctypes as C
 
 import numpy as np
@@ -10,7 +10,7 @@ from helpers import jittered_lattice
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,kernels", [(20, 15, 2), (300, 300, 3)])  # one launch, two launches
+@pytest.mark.parametrize("nx,ny,kernels", [(20, 15, 1), (33, 32, 2), (300, 300, 3)])  # one cluster, one launch, two launches
 def test_kernels_of_a_host_step(cglib, nx, ny, kernels):
     import torch
     import cellgpu_b200 as cg
