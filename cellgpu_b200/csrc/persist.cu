@@ -681,7 +681,8 @@ constexpr int PERSIST_CLUSTER = 16;
 constexpr int PERSIST_THREAD_CELLS = 192;
 
 // One block per SM at most, and no more blocks than the cells fill. Calls that run at the same time on
-// other streams take their share of the SMs: grids that fill the GPU would take turns. us per step or
+// other streams take their share of the SMs, what small ones leave included: grids that fill the GPU would
+// take turns. us per step or
 // iteration of all of M systems in M threads, full grids / shared ones / graphs:
 //   FIRE 16384 cells  M = 2  42 / 31 / 51    4   83 / 44 /  72    8  163 /  58 / 122
 //   FIRE 65536        M = 2  55 / 48 / 67    4  108 / 90 /  98    8  219 / 151 / 196
@@ -689,8 +690,8 @@ constexpr int PERSIST_THREAD_CELLS = 192;
 //   SPP  65536        M = 2  58 / 48 / 69    4  116 / 82 /  99    8  233 / 147 / 194
 static int persist_grid(const cg_system *s)
 {
-    const int share = s->in_run ? std::max(1, s->sms / (1 + running_streams.others(s))) : s->sms;
-    return std::max(1, std::min(share, nblk(s->N, cg::PERSIST_WPB * GPW)));
+    const int per_sm = cg::PERSIST_WPB * GPW;
+    return std::max(1, std::min(s->in_run ? running_streams.share(s, per_sm) : s->sms, nblk(s->N, per_sm)));
 }
 
 // Cells above which k_spp integrates after the tail, at full occupancy (the tail has 16 warps per SM): a

@@ -427,13 +427,29 @@ static int dalloc(cg_system *s, T **p, size_t count)
 // on one stream follow one another anyway): the launch forms that hold whole SMs (persist.cu) ask how
 // many others there are, which changes no result. (Never destroyed: other threads may outlive exit.)
 struct StreamUse {
+    struct Use {
+        int systems, cells;  // cells: of its largest system
+    };
     std::mutex m;
-    std::map<std::pair<int, cudaStream_t>, int> n;  // by device and stream
+    std::map<std::pair<int, cudaStream_t>, Use> n;  // by device and stream
     void add(const cg_system *s, int d)
     {
         std::lock_guard<std::mutex> lock(m);
-        const auto it = n.emplace(std::make_pair(s->device, s->stream), 0).first;
-        if ((it->second += d) == 0) n.erase(it);
+        const auto it = n.emplace(std::make_pair(s->device, s->stream), Use{0, 0}).first;
+        it->second.cells = std::max(it->second.cells, s->N);
+        if ((it->second.systems += d) == 0) n.erase(it);
+    }
+    // SMs left for s when each of the other streams has those that its cells fill (cells_per_sm each), but
+    // at most an equal share
+    int share(const cg_system *s, int cells_per_sm)
+    {
+        std::lock_guard<std::mutex> lock(m);
+        int k = 1, left = s->sms;
+        for (const auto &e : n) k += e.first.first == s->device && e.first.second != s->stream;
+        for (const auto &e : n)
+            if (e.first.first == s->device && e.first.second != s->stream)
+                left -= std::min(s->sms / k, nblk(e.second.cells, cells_per_sm));
+        return std::max(1, left);
     }
     int others(const cg_system *s)
     {
